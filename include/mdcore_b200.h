@@ -627,7 +627,8 @@ int engine_cuda_setwindow(struct engine *e, int window);
  * configuration and replays the graph from then on; a new configuration (other slot
  * count, largest cell, buffers, launch shape) is captured anew. */
 int engine_cuda_graph(struct engine *e, int enable);
-/* Persistent sweep shape: lane layout 0 = one i particle per lane (32 per warp, the
+/* Shape of the persistent sweep over the task queue (and the choice of that queue form, see
+ * engine_cuda_autotune): lane layout 0 = one i particle per lane (32 per warp, the
  * default), 1 = a tile of 8 i particles x 4 j columns per warp; stages = 1 or 2 staging
  * buffers per worker warp (2: the next task's bulk copies land while the warp sweeps the
  * current one; not with occupancy 768); occupancy = resident threads per SM the kernel's
@@ -635,9 +636,19 @@ int engine_cuda_graph(struct engine *e, int enable);
  * pair set. */
 int engine_cuda_setlayout(struct engine *e, int layout, int stages, int occupancy);
 /* Times every persistent launch shape (2, 4, 8 worker warps per block x lane layout x
- * staging buffers x occupancy, window 4) on the resident particles (uploaded first if none
- * are) and keeps the fastest; returns the chosen shape and its median device time (sort +
- * sweep).  Results stay resident. */
+ * staging buffers x occupancy, window 4) of the task-queue form on the resident particles
+ * (uploaded first if none are) and keeps the fastest; for systems with one table for every
+ * pair of types, or with tables that do not fit in shared memory, also the cell form (units of
+ * up to 24 or 32 particles of a cell against all its neighbours at once, no sort).  Returns
+ * the best queue shape and the median device time of what was kept.  Results stay resident.
+ * Both forms give the same pair, exclusion and candidate counts and forces within FP32
+ * rounding of their sums.  Time steps run the cell form only with one table (elsewhere
+ * trajectories amplify the other order of sums).  Passing the returned shape to
+ * engine_cuda_setlayout keeps the choice; any other shape, or a queue order given afterwards
+ * (engine_cuda_setorder, engine_sched_order, engine_sched_apply), selects the queue form.
+ * Without the autotuner: the queue form, and for force evaluations of systems whose tables do
+ * not fit in shared memory the cell form; the environment variable MDB_SWEEP_FORM (queue,
+ * cells, cells24), read when the device state is built, overrides, for time steps too. */
 int engine_cuda_autotune(struct engine *e, int reps, int *warps, int *layout, int *stages, int *occupancy,
                          float *ms);
 

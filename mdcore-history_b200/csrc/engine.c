@@ -465,7 +465,7 @@ int engine_step_host(struct engine *e) {
     e->time += 1;
     if (space_shuffle(s) < 0) return engine_error(engine_err_space);
     /* space_prepare's zeroing and the force evaluation in one pass over the particles */
-    if (engine_nonbond_cuda_fresh(e) < 0) return engine_error(engine_err_cuda);
+    if (nb_nonbond_step(e) < 0) return engine_error(engine_err_cuda);
     s->epot += s->epot_nonbond;
     if (engine_advance(e) < 0) return engine_error(engine_err);
     /* Resolve the rigid constraints (src/engine.c:2196-2231). */

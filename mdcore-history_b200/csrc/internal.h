@@ -28,6 +28,8 @@ double nb_ewald(double r, double kappa);
 /* Device side (nonbond.cu, rigid.cu). */
 int nb_device_free(struct engine *e);
 int rigid_device_free(struct engine *e);
+/* engine_nonbond_cuda_fresh as part of a host-threaded time step (the resident steps' form). */
+int nb_nonbond_step(struct engine *e);
 /* Zeroes forces and energies of every cell of s (host threads over ranges of cells). */
 void nb_zero_cells(struct space *s);
 /* Calls fn(ctx, part, begin, end) over contiguous ranges of [0, n) of at least `grain`

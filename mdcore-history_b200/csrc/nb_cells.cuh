@@ -1,0 +1,43 @@
+// Interface of the cell sweep (nb_cells.cu): its launch parameters, shared-memory sizes and
+// unit bound.
+#pragma once
+#include "nb_device.cuh"
+
+namespace nb {
+
+constexpr int kCellTasks = 31;           // tasks of one cell at most (one lane each)
+constexpr int kCellSlotBits = 27;        // bits of a slot number in a list entry, its task above
+
+struct CellParams {
+    Params p;
+    const int2* units;          // cell, strip | strips << 8 | share << 16 | shares << 24
+    const int* nunits;
+    int* head;                  // queue head
+    const int* toff;            // tasks of cell c (as its ci): [toff[c], toff[c + 1])
+    const TaskRec* tasks;
+    const float4* tshift;
+    const float2* cscale;       // sort scale and bias per cell (candidate counts)
+    const int* count_cand;      // nonzero: count the sorted sweep's candidates
+    int copies;                 // interleaved copies of the tables in shared memory
+    float axes[13][3];          // sort axes (candidate counts)
+    float neg_zero = -0.0f;     // square2's addend, a value the assembler does not know
+};
+
+// Most units of nslots particle slots in ncells cells of at most cap particles and maxtasks
+// tasks each.
+size_t cell_units_bound(size_t nslots, int ncells, int cap, int maxtasks);
+// Worker warps per block, interleaved table copies and shared memory for tables of ncoef floats
+// (0: read from global memory), npots tables and mt types; false when they do not fit.
+bool cell_sweep_shape(int rows, int ncoef, int npots, int mt, int* nw, int* copies, size_t* smem);
+
+// rows: i particles of a unit at most, 24 or 32.  Clears the queue words (queue head, number of units), lists the units of the cells' current
+// counts and sweeps them: nw warps per block, one block per SM.  tab: table mode (kTabShared,
+// kTabOne, kTabGlobal).  units has room for units_cap.  The kernels' attributes are set unless
+// the stream is being captured.
+cudaError_t launch_cell_sweep(const CellParams& C, int ncells, int rows, int2* units, size_t units_cap, bool has_excl,
+                              int tab, int nw, size_t smem, int grid, bool capturing, cudaStream_t s);
+
+// Counts the sorted sweep's candidates when *C.count_cand (one block per SM).
+cudaError_t launch_cell_count(const CellParams& C, int grid, cudaStream_t s);
+
+}  // namespace nb

@@ -247,7 +247,7 @@ __device__ __forceinline__ void sort_large_cell(const float4* __restrict__ xs, u
     }
 }
 
-__global__ void __launch_bounds__(kSortWarps * 32, 3) sort_cells(const float4* __restrict__ xq, const int* __restrict__ cstart,
+static __global__ void __launch_bounds__(kSortWarps * 32, 3) sort_cells(const float4* __restrict__ xq, const int* __restrict__ cstart,
                                                               const int* __restrict__ ccount,
                                                               const unsigned* __restrict__ cmask,
                                                               unsigned* __restrict__ keys,
@@ -416,7 +416,7 @@ __device__ __forceinline__ void add_task_force(const Params& P, size_t slot, flo
 
 // FP32 accumulation: the float forces of every slot into the fixed-point forces (which hold
 // nothing else yet), for the update and the readback.
-__global__ void __launch_bounds__(256) force32_to_fixed(const float* __restrict__ f32, unsigned long long* __restrict__ force,
+static __global__ void __launch_bounds__(256) force32_to_fixed(const float* __restrict__ f32, unsigned long long* __restrict__ force,
                                                         size_t n, unsigned long long* __restrict__ acc,
                                                         const unsigned long long* __restrict__ abort) {
     if (step_aborted(abort)) return;

@@ -151,7 +151,7 @@ __device__ __forceinline__ int block_scan_flag(int flag, int& excl, int* warp_to
     return total;
 }
 
-__global__ void __launch_bounds__(kQueueBlock) queue_count(const int* __restrict__ order, const TaskRec* __restrict__ tasks,
+static __global__ void __launch_bounds__(kQueueBlock) queue_count(const int* __restrict__ order, const TaskRec* __restrict__ tasks,
                                                            const int* __restrict__ ccount, int ntasks, int* __restrict__ bsum) {
     __shared__ int warp_tot[33];
     const int q = blockIdx.x * kQueueBlock + threadIdx.x;
@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(kQueueBlock) queue_count(const int* __restrict
     if (threadIdx.x == 0) bsum[blockIdx.x] = total;
 }
 
-__global__ void __launch_bounds__(kQueueBlock) queue_offsets(int* __restrict__ bsum, int nblocks, int* __restrict__ qcount) {
+static __global__ void __launch_bounds__(kQueueBlock) queue_offsets(int* __restrict__ bsum, int nblocks, int* __restrict__ qcount) {
     __shared__ int warp_tot[33];
     int run = 0;
     for (int base = 0; base < nblocks; base += kQueueBlock) {
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kQueueBlock) queue_offsets(int* __restrict__ b
     if (threadIdx.x == 0) *qcount = run;
 }
 
-__global__ void __launch_bounds__(kQueueBlock) queue_scatter(const int* __restrict__ order, const TaskRec* __restrict__ tasks,
+static __global__ void __launch_bounds__(kQueueBlock) queue_scatter(const int* __restrict__ order, const TaskRec* __restrict__ tasks,
                                                              const int* __restrict__ ccount, int ntasks,
                                                              const int* __restrict__ bsum, int* __restrict__ queue) {
     __shared__ int warp_tot[33];

@@ -33,6 +33,7 @@
 #include "mdcore_b200.h"
 #include "internal.h"
 #include "nb_tuned.cuh"
+#include "nb_cells.cuh"
 #include "nb_resident.cuh"
 #include "host_pool.h"
 
@@ -46,6 +47,8 @@ struct NbState {
     cudaStream_t own_stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;       // around sort + sweep
     cudaEvent_t evs0 = nullptr, evs1 = nullptr;     // around the sweep kernel alone
+    cudaStream_t side_stream = nullptr;    // the cell form's candidate count, beside its sweep
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // engines served by this state and their offsets in the global cell / id numbering
     std::vector<struct engine*> engines;
     std::vector<int> cell_off, id_off;
@@ -74,7 +77,26 @@ struct NbState {
     float* d_qid = nullptr;        // charges by global id (explicit electrostatics)
     std::vector<float> h_qid;
     bool one_pot = false;           // every type pair uses table 0 (no per-pair lookup)
-    int plain = 0;                 // 1: one CTA per task (the plain form); 0: persistent queue
+    int plain = 0;                 // 1: one CTA per task (the plain form); 0: persistent
+    // The persistent evaluation's form: units of one cell (nb_cells.cuh) wherever the cells'
+    // task lists fit it and nothing asks for the task queue (queue_form), see use_cells.
+    bool cells_ok = false;
+    bool queue_form = false;
+    bool cells_forced = false;     // MDB_SWEEP_FORM=cells: time steps of every system too
+    bool stepping = false;         // a host-buffer evaluation is part of a time step
+    int cell_rows = 32;            // i particles of a unit of the cell form (24 or 32)
+    bool tuned = false;            // autotuned: tuned_shape, tuned_cells are its choice
+    bool tuned_cells = false;
+    int tuned_shape[4] = {0, 0, 0, 0};
+    int max_cell_tasks = 0;
+    float axes[13][3] = {};        // the sort axes
+    int* d_toff = nullptr;         // tasks by their i cell: [toff[c], toff[c + 1]) of d_ctasks, d_cshift
+    TaskRec* d_ctasks = nullptr;
+    float4* d_cshift = nullptr;
+    int2* d_units = nullptr;       // units of the evaluation, their number and the queue head
+    size_t units_cap = 0;
+    int* d_unit_words = nullptr;   // queue head, units, count candidates (resident steps), 1
+    bool keys_stale = true;        // the host-path / resident sort keys are not the last evaluation's
     int fp32acc = 0;               // plain form: forces accumulated in FP32 (float atomics)
     float* d_force32 = nullptr;    // float forces of FP32 accumulation (3 per slot)
     size_t force32_slots = 0;
@@ -663,6 +685,107 @@ int launch_tuned(NbState* st, const Params& P, int cap4) {
     return st->layout ? launch_tuned_lay<1>(st, T, cap, smem, nw) : launch_tuned_lay<0>(st, T, cap, smem, nw);
 }
 
+// Test hook state (engine_cuda_copytimeout_test) by device: the hook is about the queue
+// form's staging copies, so evaluations with it on run that form.
+constexpr int kHookDevices = 64;
+std::atomic<int> copy_hook[kHookDevices];
+
+// Whether an evaluation runs in the cell form: not when the queue form is asked for (a launch
+// shape, or a queue order given after the autotuner), when per-task clocks are recorded, for
+// the unsorted sweep (its candidates are all pairs) or with a Verlet skin (its keys are kept
+// between steps and bound the sweep).  Time steps (steps) of systems of several tables stay in
+// the queue form: the two forms add a particle's pair forces in another order, and over some
+// hundred steps of such systems (close contacts of a random vapour, truncated charges, the
+// constraint iterations) that last bit grows to per mille of the velocities, as it does
+// between the queue form's own lane layouts; a single table's trajectories keep five digits.
+bool use_cells(const NbState* st, bool steps) {
+    if (!st->cells_ok || st->queue_form || st->plain || st->record_clock || st->unsorted) return false;
+    if (steps && !st->one_pot && !st->cells_forced) return false;
+    if (st->device >= 0 && st->device < kHookDevices && copy_hook[st->device].load() != 0) return false;
+    for (const struct engine* e : st->engines)
+        if (!(e->flags & engine_flag_verlet)) return true;
+    return false;
+}
+
+// Worker warps, table copies and shared memory of the cell form for the state's tables.
+bool cell_shape(const NbState* st, int* nw, int* copies, size_t* smem) {
+    return cell_sweep_shape(st->cell_rows, st->tab_global ? 0 : st->ncoef, st->tab_global ? 0 : st->npots, st->max_type, nw, copies,
+                            smem);
+}
+
+// The cell form's launches on the state's stream: the units of the cells' current counts and
+// their sweep, and beside the sweep, on a stream of its own that forks and joins here, the
+// candidate count (skipped on the device while *count_cand is 0).
+int launch_cells(NbState* st, const Params& P, const int* count_cand) {
+    CellParams C;
+    C.p = P;
+    C.units = st->d_units;
+    C.nunits = st->d_unit_words + 1;
+    C.head = st->d_unit_words;
+    C.toff = st->d_toff;
+    C.tasks = st->d_ctasks;
+    C.tshift = st->d_cshift;
+    C.cscale = st->d_cscale;
+    C.count_cand = count_cand;
+    std::memcpy(C.axes, st->axes, sizeof(C.axes));
+    int nw = 0;
+    size_t smem = 0;
+    cell_shape(st, &nw, &C.copies, &smem);
+    CU(cudaEventRecord(st->ev_fork, st->stream));
+    CU(cudaStreamWaitEvent(st->side_stream, st->ev_fork, 0));
+    CU(launch_cell_sweep(C, st->ncells, st->cell_rows, st->d_units, st->units_cap, st->has_excl,
+                         st->tab_global ? kTabGlobal : st->one_pot ? kTabOne : kTabShared, nw, smem, st->sm_count,
+                         st->capturing, st->stream));
+    CU(launch_cell_count(C, st->sm_count, st->side_stream));
+    CU(cudaEventRecord(st->ev_join, st->side_stream));
+    CU(cudaStreamWaitEvent(st->stream, st->ev_join, 0));
+    return 0;
+}
+
+// The tasks by their i cell, built when the cell form first runs (directly: captures follow a
+// direct launch).
+int build_cell_tasks(NbState* st) {
+    if (st->d_toff != nullptr) return 0;
+    const int nc = st->ncells, nt = st->ntasks;
+    std::vector<TaskRec> tasks(nt), ct(nt);
+    std::vector<float4> shift(nt), cs(nt);
+    std::vector<int> toff(nc + 1, 0);
+    CU(cudaMemcpy(tasks.data(), st->d_tasks, sizeof(TaskRec) * nt, cudaMemcpyDeviceToHost));
+    CU(cudaMemcpy(shift.data(), st->d_tshift, sizeof(float4) * nt, cudaMemcpyDeviceToHost));
+    for (int t = 0; t < nt; t++) toff[tasks[t].ci + 1]++;
+    for (int c = 0; c < nc; c++) toff[c + 1] += toff[c];
+    std::vector<int> at(toff.begin(), toff.end());
+    for (int t = 0; t < nt; t++) {
+        const int k = at[tasks[t].ci]++;
+        ct[k] = tasks[t];
+        cs[k] = shift[t];
+    }
+    if (dev_alloc(&st->d_ctasks, nt) || dev_alloc(&st->d_cshift, nt) || dev_alloc(&st->d_toff, nc + 1))
+        return engine_err_cuda;
+    CU(cudaMemcpy(st->d_ctasks, ct.data(), sizeof(TaskRec) * nt, cudaMemcpyHostToDevice));
+    CU(cudaMemcpy(st->d_cshift, cs.data(), sizeof(float4) * nt, cudaMemcpyHostToDevice));
+    CU(cudaMemcpy(st->d_toff, toff.data(), sizeof(int) * toff.size(), cudaMemcpyHostToDevice));
+    return 0;
+}
+
+// Room for the units of `slots` particle slots in cells of at most cap4, grown on a direct
+// launch (a captured one has been preceded by a direct one of the same sizes).
+int reserve_units(NbState* st, size_t slots, int cap4) {
+    const size_t need = cell_units_bound(slots, st->ncells, cap4, st->max_cell_tasks);
+    if (need <= st->units_cap) return 0;
+    if (st->capturing) {
+        errs_register(engine_err_cuda, "Unit list too small inside a stream capture.", __LINE__, __func__, __FILE__);
+        return engine_err = engine_err_cuda;
+    }
+    if (st->d_units) CU(cudaFree(st->d_units));
+    st->d_units = nullptr;
+    st->units_cap = 0;
+    if (dev_alloc(&st->d_units, need)) return engine_err_cuda;
+    st->units_cap = need;
+    ++st->buf_gen;
+    return 0;
+}
+
 // Records an event; inside a stream capture as an external record node, so that replaying
 // the graph records it again (a plain record would stay internal to the graph).
 int record_event(NbState* st, cudaEvent_t ev) {
@@ -688,6 +811,7 @@ struct DevView {
     const unsigned long long* abort = nullptr;   // resident steps: the step's abort word
     const int* rebuild = nullptr;                // Verlet skin: sort only when *rebuild
     const int* cell_mdx = nullptr;               // Verlet skin: displacements in key units
+    bool resident = false;
 };
 
 DevView host_view(const NbState* st) {
@@ -722,9 +846,17 @@ int issue_kernels(NbState* st, const DevView& V, bool span = true) {
         if (rc == 0 && span) rc = record_event(st, st->ev1);
         return rc;
     }
-    int rc0 = launch_sort(V.xq, V.cstart, V.ccount, st->d_cmask, V.keys, st->d_cscale, st->ncells, V.cpc, cap,
-                          st->d_acc, V.abort, st->capturing, st->stream, V.rebuild);
-    if (rc0 < 0) return rc0;
+    const bool cells = use_cells(st, V.resident || st->stepping);
+    st->keys_stale = cells;
+    if (!cells) {
+        const int rc0 = launch_sort(V.xq, V.cstart, V.ccount, st->d_cmask, V.keys, st->d_cscale, st->ncells, V.cpc, cap,
+                                    st->d_acc, V.abort, st->capturing, st->stream, V.rebuild);
+        if (rc0 < 0) return rc0;
+    } else {
+        int rc0 = st->capturing ? 0 : build_cell_tasks(st);
+        if (rc0 == 0) rc0 = reserve_units(st, V.slots, cap);
+        if (rc0 < 0) return rc0;
+    }
 
     Params P;
     P.xq = V.xq;
@@ -779,7 +911,11 @@ int issue_kernels(NbState* st, const DevView& V, bool span = true) {
     }
     int rc = record_event(st, st->evs0);
     if (rc < 0) return rc;
-    rc = st->plain ? launch_plain(st, P, cap) : launch_tuned(st, P, cap);
+    // candidates: every host evaluation; of resident steps the last of a call (words[2])
+    if (cells)
+        rc = launch_cells(st, P, st->d_unit_words + (V.resident ? 2 : 3));
+    else
+        rc = st->plain ? launch_plain(st, P, cap) : launch_tuned(st, P, cap);
     if (rc < 0) return rc;
     rc = record_event(st, st->evs1);
     if (rc < 0) return rc;
@@ -794,6 +930,17 @@ int issue_kernels(NbState* st, const DevView& V, bool span = true) {
 }
 
 int issue_kernels(NbState* st) { return issue_kernels(st, host_view(st)); }
+
+// The sort keys of the uploaded particles, for readers of the keys after evaluations in the
+// cell form, which needs none.
+int sort_keys(NbState* st, const DevView& V) {
+    if (V.cap4 == 0) return 0;
+    const int rc = launch_sort(V.xq, V.cstart, V.ccount, st->d_cmask, V.keys, st->d_cscale, st->ncells, V.cpc, V.cap4,
+                               st->d_acc, nullptr, false, st->stream);
+    if (rc == 0) st->keys_stale = false;
+    return rc;
+}
+int sort_host_keys(NbState* st) { return sort_keys(st, host_view(st)); }
 
 void drop_graph(NbState* st) {
     if (st->graph_exec) cudaGraphExecDestroy(st->graph_exec);
@@ -816,6 +963,7 @@ long long launch_key(const NbState* st) {
     k = k * 3 + st->plain;
     k = k * 3 + st->record_clock;
     k = k * 2 + st->fp32acc;
+    k = k * 4 + (use_cells(st, st->stepping) ? st->cell_rows / 8 - 2 : 0);
     return k;
 }
 
@@ -827,6 +975,7 @@ int launch_kernels(NbState* st) {
     const long long key = launch_key(st);
     if (st->graph_exec != nullptr && st->graph_key == key) {
         CU(cudaGraphLaunch(st->graph_exec, st->stream));
+        st->keys_stale = use_cells(st, st->stepping);
         return 0;
     }
     if (st->prepared_key != key) {
@@ -949,7 +1098,8 @@ void state_free(NbState* st) {
                    st->d_cscale, st->d_acc, st->d_cell_epot, st->d_tasks, st->d_tshift, st->d_coef, st->d_potinfo,
                    st->d_potn, st->d_potidx, st->d_emask, st->d_exoff, st->d_exlist, st->d_order,
                    st->d_counter, st->d_task_clock, st->d_task_sm, st->d_forcef, st->d_queue,
-                   st->d_qcount, st->d_bsum, st->d_qid, st->d_force32, st->r_elog, st->r_eacc};
+                   st->d_qcount, st->d_bsum, st->d_qid, st->d_force32, st->r_elog, st->r_eacc, st->d_toff,
+                   st->d_ctasks, st->d_cshift, st->d_units, st->d_unit_words};
     for (void* p : dev) cudaFree(p);
     void* host[] = {st->h_xq, st->h_pid, st->h_cstart, st->h_force, st->h_cell_epot, st->h_acc};
     for (void* p : host) cudaFreeHost(p);
@@ -957,6 +1107,9 @@ void state_free(NbState* st) {
     if (st->ev1) cudaEventDestroy(st->ev1);
     if (st->evs0) cudaEventDestroy(st->evs0);
     if (st->evs1) cudaEventDestroy(st->evs1);
+    if (st->ev_fork) cudaEventDestroy(st->ev_fork);
+    if (st->ev_join) cudaEventDestroy(st->ev_join);
+    if (st->side_stream) cudaStreamDestroy(st->side_stream);
     for (cudaEvent_t ev : st->chunk_ev) cudaEventDestroy(ev);
     if (st->own_stream) cudaStreamDestroy(st->own_stream);
     sched_free(st->sched);
@@ -1012,6 +1165,9 @@ int load_state(NbState* st) {
     CU(cudaEventCreate(&st->ev1));
     CU(cudaEventCreate(&st->evs0));
     CU(cudaEventCreate(&st->evs1));
+    CU(cudaStreamCreateWithFlags(&st->side_stream, cudaStreamNonBlocking));
+    CU(cudaEventCreateWithFlags(&st->ev_fork, cudaEventDisableTiming));
+    CU(cudaEventCreateWithFlags(&st->ev_join, cudaEventDisableTiming));
     CU(cudaDeviceGetAttribute(&st->sm_count, cudaDevAttrMultiProcessorCount, st->device));
     nb_sweep_scales(&e0->s, &st->bias, &st->dscale, &st->dmaxdist);
     const float cutf = (float)e0->s.cutoff;
@@ -1019,9 +1175,8 @@ int load_state(NbState* st) {
     st->cut2s = (float)e0->s.cutoff2;
     st->unsorted = (e0->flags & engine_flag_unsorted) ? 1 : 0;
 
-    float axes[13][3];
-    for (int sid = 0; sid < 13; sid++) sort_axis(sid, axes[sid]);
-    CU(cudaMemcpyToSymbol(c_axes, axes, sizeof(axes)));
+    for (int sid = 0; sid < 13; sid++) sort_axis(sid, st->axes[sid]);
+    CU(cudaMemcpyToSymbol(c_axes, st->axes, sizeof(st->axes)));
 
     // Potential tables: one copy of every distinct table, type pair -> table index.
     std::vector<struct potential*> uniq;
@@ -1116,6 +1271,26 @@ int load_state(NbState* st) {
             cost[t0 + t] = task_weight(r.sid, s->cells[r.ci - c0].count, s->cells[r.cj - c0].count);
         }
         t0 += s->nr_tasks;
+    }
+    {   // what decides whether the cell form can and does run
+        std::vector<int> per_cell(st->ncells + 1, 0);
+        for (int t = 0; t < ntasks; t++) per_cell[tasks[t].ci]++;
+        st->max_cell_tasks = *std::max_element(per_cell.begin(), per_cell.end());
+        if (dev_alloc(&st->d_unit_words, 4)) return engine_err_cuda;
+        const int words[4] = {0, 0, 1, 1};
+        CU(cudaMemcpy(st->d_unit_words, words, sizeof(words), cudaMemcpyHostToDevice));
+        int nw = 0, copies = 0;
+        size_t smem = 0;
+        st->cells_ok = st->max_cell_tasks <= kCellTasks && cell_shape(st, &nw, &copies, &smem) && nw >= 4;
+        // Without the autotuner: the cell form (24 rows) where the tables are read from global
+        // memory (many type pairs, explicit charges; force evaluation of solvated chains, 12,400
+        // atoms: sweep 0.55 -> 0.27 ms), else the task queue, which small systems finish sooner (argon, 8,788 atoms:
+        // 0.058 against 0.066 ms).  Properties of the engines' tables, so an engine runs the same
+        // form alone and in a batch.  MDB_SWEEP_FORM=queue, cells or cells24 overrides.
+        const char* form = std::getenv("MDB_SWEEP_FORM");
+        st->cells_forced = form && std::strncmp(form, "cells", 5) == 0;
+        st->queue_form = form ? std::strncmp(form, "cells", 5) != 0 : !st->tab_global;
+        st->cell_rows = form ? (std::strcmp(form, "cells24") == 0 ? 24 : 32) : st->tab_global ? 24 : 32;
     }
     if (dev_alloc(&st->d_tasks, tasks.size()) || dev_alloc(&st->d_tshift, tshift.size())) return engine_err_cuda;
     CU(cudaMemcpy(st->d_tasks, tasks.data(), tasks.size() * sizeof(TaskRec), cudaMemcpyHostToDevice));
@@ -1364,6 +1539,14 @@ int st_nonbond(NbState* st, bool fresh = false) {
     return st_unload_parts(st, fresh);
 }
 
+// The force evaluation of a host-threaded time step: in the form of the resident steps.
+int st_nonbond_step(NbState* st) {
+    st->stepping = true;
+    const int rc = st_nonbond(st, true);
+    st->stepping = false;
+    return rc;
+}
+
 int st_setstream(NbState* st, void* stream) {
     CU(cudaSetDevice(st->device));
     CU(cudaStreamSynchronize(st->stream));
@@ -1406,6 +1589,7 @@ int st_autotune(NbState* st, int reps, int* warps_out, int* layout_out, int* sta
     const bool graph = st->use_graph;
     st->use_graph = false;
     st->plain = 0;
+    st->queue_form = true;
     // warps, layout, stages, threads per SM (window 4: the 8-step window was never the
     // fastest shape)
     static const int shapes[][4] = {
@@ -1447,8 +1631,47 @@ int st_autotune(NbState* st, int reps, int* warps_out, int* layout_out, int* sta
     st->stages = shapes[best][2];
     st->occupancy = shapes[best][3];
     st->window = 4;
+    // The cell form with units of 32 and of 24 rows, for the systems whose steps or default
+    // evaluations may run it; kept when it beats the queue form's best (whose shape is the one
+    // returned).  It is timed without its candidate count, which
+    // resident steps take once per call only.
+    st->queue_form = false;
+    int best_rows = 0;
+    if (use_cells(st, false) && (st->one_pot || st->tab_global || st->cells_forced)) {
+        cudaError_t err = cudaMemsetAsync(st->d_unit_words + 3, 0, sizeof(int), st->stream);
+        int rc = 0;
+        for (int rows = 32; rows >= 24 && rc == 0 && err == cudaSuccess; rows -= 8) {
+            st->cell_rows = rows;
+            std::vector<float> t;
+            for (int r = 0; r <= reps && rc == 0 && err == cudaSuccess; r++) {
+                rc = st_resident(st);
+                if (rc < 0) break;
+                err = cudaEventSynchronize(st->ev1);
+                float ms = 0.f;
+                if (err == cudaSuccess) err = cudaEventElapsedTime(&ms, st->ev0, st->ev1);
+                if (r > 0) t.push_back(ms);
+            }
+            if (rc < 0 || err != cudaSuccess) break;
+            std::sort(t.begin(), t.end());
+            if (t[t.size() / 2] < best_ms) {
+                best_ms = t[t.size() / 2];
+                best_rows = rows;
+            }
+        }
+        if (err == cudaSuccess) err = cudaMemsetAsync(st->d_unit_words + 3, 1, sizeof(int), st->stream);
+        if (rc < 0 || err != cudaSuccess) {
+            st->use_graph = graph;
+            CU(err);
+            return rc;
+        }
+    }
+    st->queue_form = best_rows == 0;
+    if (best_rows) st->cell_rows = best_rows;
+    st->tuned = true;
+    st->tuned_cells = !st->queue_form;
+    for (int k = 0; k < 4; k++) st->tuned_shape[k] = shapes[best][k];
     st->use_graph = graph;
-    const int rc = st_resident(st);           // leave the chosen shape's results resident
+    const int rc = st_resident(st);           // leave the chosen form's results resident
     if (rc < 0) return rc;
     if (warps_out) *warps_out = st->warps;
     if (layout_out) *layout_out = st->layout;
@@ -1740,6 +1963,7 @@ int res_alloc(NbState* st, int capc, int mcap, long long n) {
     st->mcap = mcap;
     st->res_nparts = n;
     const size_t slots = (size_t)nc * st->capc;
+    if (slots >> kCellSlotBits) st->cells_ok = false;      // beyond the cell form's slot numbers
     for (int q = 0; q < 2; q++) {
         CU(cudaMalloc(&st->r_xq[q], sizeof(float4) * slots));
         CU(cudaMalloc(&st->r_v[q], sizeof(float4) * slots));
@@ -1989,6 +2213,7 @@ int res_issue_step(NbState* st) {
     V.abort = st->r_status;
     V.slots = (size_t)st->ncells * st->capc;
     V.cap4 = st->capc;
+    V.resident = true;
     V.cpc = st->res_nparts <= 32LL * st->ncells ? kSortWarps : 1;   // one warp per small cell
     rc = issue_kernels(st, V, false);
     if (rc < 0) return rc;
@@ -2098,6 +2323,7 @@ long long res_key(const NbState* st) {
     k = k * 2 + (st->sd_gamma > 0.f);
     k = k * 2 + (st->elog_cap > 0);
     k = k * 2 + st->verlet;
+    k = k * 4 + (use_cells(st, true) ? st->cell_rows / 8 - 2 : 0);
     return k;
 }
 
@@ -2107,6 +2333,10 @@ long long res_key(const NbState* st) {
 // ones replay.
 int res_issue_steps(NbState* st, int nsteps) {
     for (int k = 0; k < nsteps; k++) {
+        // The candidate count of a step can be read only after the last step of a call (the cell
+        // form spends extra work on it).
+        if (k == 0 || k == nsteps - 1)
+            CU(cudaMemsetAsync(st->d_unit_words + 2, k == nsteps - 1, sizeof(int), st->stream));
         bool refine = false;
         for (struct engine* e : st->engines) {
             e->time += 1;
@@ -2119,6 +2349,7 @@ int res_issue_steps(NbState* st, int nsteps) {
             if (rc < 0) return rc;
         } else if (st->rgraph_exec[side] != nullptr && st->rgraph_key[side] == key) {
             CU(cudaGraphLaunch(st->rgraph_exec[side], st->stream));
+            st->keys_stale = use_cells(st, true);
         } else if (st->rprepared[side] != key) {
             const int rc = res_issue_step(st);
             if (rc < 0) return rc;
@@ -2504,6 +2735,9 @@ static int st_setlayout(NbState* st, int layout, int stages, int occupancy) {
     st->layout = layout;
     st->stages = stages;
     st->occupancy = occupancy;
+    // A shape is one of the queue form; the shape the autotuner returned stands for its choice.
+    st->queue_form = !(st->tuned_cells && layout == st->tuned_shape[1] && stages == st->tuned_shape[2] &&
+                       occupancy == st->tuned_shape[3]);
     return 0;
 }
 
@@ -2552,6 +2786,7 @@ extern "C" int engine_cuda_copytimeout_test(struct engine* e, int enable) {
     CU(cudaSetDevice(st->device));
     CU(cudaStreamSynchronize(st->stream));
     CU(cudaMemcpyToSymbol(c_skip_copies, &enable, sizeof(enable)));
+    if (st->device >= 0 && st->device < kHookDevices) copy_hook[st->device].store(enable);
     return 0;
 }
 
@@ -2677,6 +2912,13 @@ extern "C" int engine_nonbond_cuda_fresh(struct engine* e) {
     return st_nonbond(state(e), true);
 }
 
+// The force evaluation of engine_step_host (no error stack entry of its own).
+extern "C" int nb_nonbond_step(struct engine* e) {
+    if (e == nullptr) return engine_err_null;
+    if (e->cuda == nullptr && engine_cuda_load(e) < 0) return engine_err_cuda;
+    return st_nonbond_step(state(e));
+}
+
 // Sort + sweep on the particles already resident on the device (no host copies, no
 // synchronisation); results stay on the device until engine_cuda_unload_parts.
 extern "C" int engine_nonbond_cuda_resident(struct engine* e) {
@@ -2800,6 +3042,9 @@ void copy_shape(NbState* c, const NbState* st) {
     c->layout = st->layout;
     c->stages = st->stages;
     c->occupancy = st->occupancy;
+    c->queue_form = st->queue_form || !st->cells_ok;
+    c->cell_rows = st->cell_rows;
+    c->cells_forced = st->cells_forced;
     c->use_graph = st->use_graph;
     c->plain = st->plain;
     c->fp32acc = st->fp32acc;
@@ -2959,6 +3204,11 @@ extern "C" int engine_cuda_getsort(struct engine* e, int cid, unsigned int* keys
     int n = s->cells[cid].count, pad = (n + 3) & ~3;
     if (size < 13 * n) return engine_err_range;
     std::vector<unsigned> buf(13 * (size_t)pad + 1);
+    CU(cudaSetDevice(st->device));
+    if (st->keys_stale && !st->res_active && st->resident_valid) {      // the cell form sorts nothing
+        const int rc = sort_host_keys(st);
+        if (rc < 0) return rc;
+    }
     CU(cudaStreamSynchronize(st->stream));
     CU(cudaMemcpy(buf.data(), st->d_keys + 13 * (size_t)st->h_cstart[cid], sizeof(unsigned) * 13 * (size_t)pad,
                   cudaMemcpyDeviceToHost));
@@ -3059,7 +3309,7 @@ extern "C" int engine_batch_step_host(struct engine_batch* b) {
         e->time += 1;
         if (space_shuffle(&e->s) < 0) return engine_err = engine_err_space;
     }
-    const int rc = st_nonbond(st, true);
+    const int rc = st_nonbond_step(st);
     if (rc < 0) return rc;
     for (struct engine* e : st->engines) {
         e->s.epot += e->s.epot_nonbond;
@@ -3223,6 +3473,9 @@ int st_setorder(NbState* st, const int* order, int n) {
     CU(cudaSetDevice(st->device));
     CU(cudaStreamSynchronize(st->stream));
     CU(cudaMemcpy(st->d_order, order, sizeof(int) * n, cudaMemcpyHostToDevice));
+    // An order is about the task queue.  Given after the autotuner it selects the queue form
+    // (in its best shape); before it, the form (and so the rounding of the forces) stays.
+    if (st->tuned) st->queue_form = true;
     return 0;
 }
 }  // namespace
@@ -3626,6 +3879,21 @@ extern "C" int engine_sched_features(struct engine* e, float* features_out, int 
     const int* cstart = res ? st->r_cstart : st->d_cstart;
     const int* ccount = res ? st->r_cnt[st->rside] : st->d_ccount;
     const unsigned* keys = res ? st->r_keys : st->d_keys;
+    if (st->keys_stale && (res || st->resident_valid)) {
+        DevView V;
+        if (res) {
+            V.xq = xq;
+            V.keys = st->r_keys;
+            V.cstart = cstart;
+            V.ccount = ccount;
+            V.cap4 = st->capc;
+            V.cpc = st->res_nparts <= 32LL * st->ncells ? kSortWarps : 1;
+        } else {
+            V = host_view(st);
+        }
+        const int rc = sort_keys(st, V);
+        if (rc < 0) return rc;
+    }
     cell_type0<<<(st->ncells + 255) / 256, 256, 0, st->stream>>>(xq, cstart, ccount, st->ncells, ss->d_ctype0);
     task_features<<<(st->ntasks + 255) / 256, 256, 0, st->stream>>>(st->d_tasks, st->ntasks, ccount, cstart, keys,
                                                                     ss->d_ctype0, 1.0f / 32.0f, ss->d_feat);

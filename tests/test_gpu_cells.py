@@ -1,0 +1,151 @@
+"""GPU tests of the cell form of the persistent evaluation (sweep_cells: units of up to 32 i
+particles of a cell against the j particles of all its tasks; MDB_SWEEP_FORM=cells selects it
+as the autotuner otherwise does): pairs, exclusions and the sorted sweep's candidate count
+exact, energy, virial and forces within the parity bounds of the oracle, at the sizes where
+its strips, lists and masks end (cells of 0 to 90 particles, a cell of 1,000, a vapour, list
+and mask exclusions, many tables), and the same results alone, in a batch,
+resident and through engine_step."""
+import numpy as np
+import pytest
+
+import mdcore_b200 as M
+import oracle as O
+import workloads as W
+from helpers import force_errors, load_golden, tables_of
+from test_gpu_edges import lj_system
+from test_gpu_parity import cells_of_every_size, cells_of_every_size_2nm
+
+pytestmark = pytest.mark.gpu
+
+
+def one_large_cell():
+    rng = np.random.default_rng(3)
+    dense = rng.uniform(0.0, 1.0, size=(1000, 3))
+    sparse = rng.uniform(0.0, 3.0, size=(200, 3))
+    return lj_system(np.concatenate([dense, sparse[(sparse >= 1.0).any(axis=1)]]), L=3.0, scale=1e-4)
+
+
+def far_exclusions():
+    base, _ = load_golden("argon_1372.npz")
+    rng = np.random.default_rng(5)
+    pairs = set()
+    while len(pairs) < 200:
+        i, j = (int(v) for v in rng.integers(0, base.n, size=2))
+        d = base.x[i] - base.x[j]
+        d -= np.round(d / base.dim) * base.dim
+        if i != j and (d ** 2).sum() < 0.8:
+            pairs.add((i, j))
+    return W.System(**{**base.__dict__, "excl": np.array(sorted(pairs), np.int32), "name": "argon-far-excl"})
+
+
+def on_cell_faces():
+    """Particles on the faces of their cells."""
+    rng = np.random.default_rng(8)
+    x = rng.uniform(0.0, 4.0, size=(1500, 3))
+    x[:300, rng.integers(0, 3)] = np.round(x[:300, 0])
+    return lj_system(np.mod(x, 4.0), L=4.0, scale=1e-4)
+
+
+SYSTEMS = {
+    "cells-0-40": cells_of_every_size,
+    "cells-0-90": cells_of_every_size_2nm,
+    "cell-1000": one_large_cell,
+    "faces": on_cell_faces,
+    "far-exclusions": far_exclusions,
+    "water": lambda: W.water_spce(11, seed=2),
+    "vapour": lambda: W.lj_slab(nx=22, nz=11, n_total=22 * 22 * 11 + 1000, box=(8.0, 8.0, 24.0), slab=4.0, seed=4),
+    "dilute-water": lambda: W.water_spce(nside=8, density=1.0, seed=3),
+    "chains": lambda: W.chains_water(nchains=4, length=20, nwater=150, box=(6.0, 6.0, 6.0), seed=2,
+                                     angles_dihedrals=False),
+    "single": lambda: lj_system(np.full((1, 3), 0.5)),
+}
+
+
+_ORACLE = {}
+
+
+@pytest.mark.parametrize("cells", ["cells", "cells24"])
+@pytest.mark.parametrize("name", SYSTEMS)
+def test_cell_form_vs_oracle_and_queue_form(name, cells, monkeypatch):
+    sysm = SYSTEMS[name]()
+    if name not in _ORACLE:
+        _ORACLE[name] = O.nonbond(sysm, tables_of(sysm))
+    o = _ORACLE[name]
+    out = {}
+    for form in (cells, "queue"):
+        monkeypatch.setenv("MDB_SWEEP_FORM", form)
+        e = M.Engine.from_system(sysm)
+        e.nonbond()
+        out[form] = e.forces(), e.stats(), [e.sortkeys(c, int((e.cells() == c).sum())) for c in (0, 1, 5)]
+        e.close()
+    f, st, keys = out[cells]
+    q = out["queue"][1]
+    assert st.status == 0
+    assert (st.pairs, st.excluded, st.candidates) == (o["pairs"], o["excluded"], q.candidates)
+    assert abs(st.epot - o["epot"]) <= 1e-6 * o["epot_abs"] and abs(st.virial - o["virial"]) <= 1e-6 * o["virial_abs"]
+    if st.pairs:
+        err = force_errors(f, o["f"])
+        assert err["global_rel"] <= 2e-6 and err["max_over_frms"] <= 2e-5, err
+    assert all(np.array_equal(a, b) for a, b in zip(keys, out["queue"][2]))     # sorted on demand
+
+
+@pytest.mark.parametrize("name", ["water", "replicas"])
+def test_cell_form_is_the_same_alone_in_a_batch_and_resident(name, monkeypatch):
+    monkeypatch.setenv("MDB_SWEEP_FORM", "cells")
+    systems = [W.with_rigid_water(W.water_spce(10), 300.0)] if name == "water" else W.argon_replicas(5, seed=9)
+    for s in systems:
+        if s.v is None:
+            s.v = W.maxwell_velocities(s, 100.0, seed=1)
+    engines = [M.Engine.from_system(s, start=False) for s in systems]
+    b = M.Batch(engines)
+    b.graph(True)
+    b.resident_begin().resident_steps(7)
+    b.resident_sync()
+    for s, r in zip(systems, engines):
+        e = M.Engine.from_system(s)
+        for _ in range(7):
+            e.step()
+        assert all(np.array_equal(x, y) for x, y in zip(e.parts(), r.parts()))
+        assert e.energies() == r.energies()
+        st = e.stats()
+        if len(systems) == 1:
+            assert st.candidates == b.stats().candidates
+        e.close()
+    b.close()
+
+
+def test_candidates_of_the_last_step_of_every_call(monkeypatch):
+    """The count is taken in the last step of a call only; it is the queue form's."""
+    sysm = W.argon_fcc(7, jitter=0.05)
+    sysm.v = W.maxwell_velocities(sysm, 150.0, seed=3)
+    got = {}
+    for form in ("cells", "queue"):
+        monkeypatch.setenv("MDB_SWEEP_FORM", form)
+        e = M.Engine.from_system(sysm)
+        e.graph(True)
+        e.resident_begin()
+        got[form] = []
+        for k in (1, 3, 1, 2):
+            e.resident_steps(k)
+            e.resident_sync()
+            got[form].append((e.stats().pairs, e.stats().candidates))
+        e.close()
+    assert got["cells"] == got["queue"]
+
+
+def test_steps_of_several_tables_keep_the_queue_form(monkeypatch):
+    """Default engines of many tables: force evaluations run the cell form, time steps (device
+    and host-threaded) give the queue form's trajectory bit for bit."""
+    sysm = W.chains_water(nchains=6, length=20, nwater=200, box=(4.0, 4.0, 4.0), seed=2, angles_dihedrals=False)
+    sysm.bonds = None
+    out = []
+    for form, host in ((None, False), (None, True), ("queue", False)):
+        if form:
+            monkeypatch.setenv("MDB_SWEEP_FORM", form)
+        e = M.Engine.from_system(sysm)
+        for _ in range(3):
+            e.step_host() if host else e.step()
+        out.append(e.parts())
+        e.close()
+    for other in out[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(out[0][:2], other[:2]))
