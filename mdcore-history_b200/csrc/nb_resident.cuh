@@ -43,9 +43,24 @@ struct ResidentCells {
 // Direction index of a cell offset (dx, dy, dz) in {-1, 0, 1}^3.
 __device__ __forceinline__ int dir_index(int dx, int dy, int dz) { return (dx + 1) * 9 + (dy + 1) * 3 + (dz + 1); }
 
-// Phase 1, one warp per cell: particles still inside [0, h) keep their order and are
-// written to the same cell of the output side; leavers go to the cell's mover list,
-// shifted into their destination cell's frame (src/space.c: x -= delta*h).
+// Per-cell kernels run with G lanes per cell: a whole warp for systems of few or large cells,
+// 8 lanes (four cells per warp) for many small ones, where a warp per cell spent its time on
+// launching blocks and on one chain of loads for a handful of particles (slab of 256,000
+// cells, 4 particles on average: split 80 -> 30 us, gather 76 -> 22 us, update 56 -> 22 us).
+template <int G>
+__device__ __forceinline__ int group_cell() {
+    return (int)((blockIdx.x * blockDim.x + threadIdx.x) / G);
+}
+template <int G>
+__device__ __forceinline__ unsigned group_bits(unsigned ballot) {
+    if constexpr (G == 32) return ballot;
+    return (ballot >> ((threadIdx.x & 31) / G * G)) & ((1u << G) - 1u);
+}
+
+// Phase 1: particles still inside [0, h) keep their order and are written to the same cell of
+// the output side; leavers go to the cell's mover list, shifted into their destination cell's
+// frame (src/space.c: x -= delta*h).
+template <int G>
 __global__ void __launch_bounds__(256) rebin_split(ResidentCells RC, const float4* __restrict__ xq,
                                                    const float4* __restrict__ v, const int* __restrict__ pid,
                                                    const int* __restrict__ count, float4* __restrict__ xq_out,
@@ -54,41 +69,43 @@ __global__ void __launch_bounds__(256) rebin_split(ResidentCells RC, const float
                                                    Mover* __restrict__ movers, unsigned long long* status,
                                                    const int* __restrict__ rebuild) {
     constexpr unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (c >= RC.ncells || *(volatile unsigned long long*)status != 0) return;
-    const int n = min(count[c], RC.capc);
+    const int gl = threadIdx.x & (G - 1);
+    const int c = group_cell<G>();
+    if (*(volatile unsigned long long*)status != 0) return;
+    const bool cell = c < RC.ncells;          // the warp's ballots need all its lanes
+    const int n = cell ? min(count[c], RC.capc) : 0;
     const size_t base = (size_t)c * RC.capc;
     // Verlet skin between rebuilds: nobody leaves (particles stay in their cells, in their
     // slots, up to half the skin outside the cell), the block is copied in order.
     const bool moving = rebuild == nullptr || *rebuild != 0;
-    const float4 h = moving ? RC.cell_h[c] : make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+    const float4 h = moving && n > 0 ? RC.cell_h[c] : make_float4(INFINITY, INFINITY, INFINITY, 0.f);
     int stays = 0, moves = 0;
-    // the next 32 particles are loaded while these are written (latency of one load, not of
-    // one per 32 particles)
+    // the next particles are loaded while these are written (latency of one load, not of one
+    // per pass)
     float4 xn = make_float4(0.f, 0.f, 0.f, 0.f), vn = xn;
     int idn = 0;
-    if (lane < n) {
-        xn = xq[base + lane];
-        vn = v[base + lane];
-        idn = pid[base + lane];
+    if (gl < n) {
+        xn = xq[base + gl];
+        vn = v[base + gl];
+        idn = pid[base + gl];
     }
-    for (int k0 = 0; k0 < n; k0 += 32) {
-        const int k = k0 + lane;
+    const int nmax = G == 32 ? n : (int)__reduce_max_sync(FULL, (unsigned)n);
+    for (int k0 = 0; k0 < nmax; k0 += G) {
+        const int k = k0 + gl;
         const bool active = k < n;
         const float4 x = xn, vv = vn;
         const int id = idn;
-        if (k + 32 < n) {
-            xn = xq[base + k + 32];
-            vn = v[base + k + 32];
-            idn = pid[base + k + 32];
+        if (k + G < n) {
+            xn = xq[base + k + G];
+            vn = v[base + k + G];
+            idn = pid[base + k + G];
         }
         const int dx = moving ? (x.x >= h.x) - (x.x < 0.0f) : 0, dy = moving ? (x.y >= h.y) - (x.y < 0.0f) : 0,
                   dz = moving ? (x.z >= h.z) - (x.z < 0.0f) : 0;
         const bool stay = active && dx == 0 && dy == 0 && dz == 0;
         const bool move = active && !stay;
-        const unsigned bs = __ballot_sync(FULL, stay), bm = __ballot_sync(FULL, move);
-        const unsigned below = (1u << lane) - 1u;
+        const unsigned bs = group_bits<G>(__ballot_sync(FULL, stay)), bm = group_bits<G>(__ballot_sync(FULL, move));
+        const unsigned below = (1u << gl) - 1u;
         if (stay) {
             const int o = stays + __popc(bs & below);
             xq_out[base + o] = x;
@@ -112,82 +129,80 @@ __global__ void __launch_bounds__(256) rebin_split(ResidentCells RC, const float
         stays += __popc(bs);
         moves += __popc(bm);
     }
-    if (lane == 0) {
+    if (gl == 0 && cell) {
         nstay[c] = stays;
         nmove[c] = min(moves, RC.mcap);
     }
 }
 
-// Phase 2, one warp per destination cell: after its stayers, the arrivals from the
-// neighbours in direction order 0..26 (a particle that moved by d arrives from the
-// neighbour at -d), each neighbour's leavers in their order; with slot_of, the slot of
-// every particle id of the cell.
+// Phase 2, the destination cells: after a cell's stayers, the arrivals from the neighbours in
+// direction order 0..26 (a particle that moved by d arrives from the neighbour at -d), each
+// neighbour's leavers in their order.  Lane g of the group owns the directions [D g, D g + D):
+// it counts its arrivals, a scan over the group gives their first slot, and it writes them.
+// With slot_of, the slot of every particle id of the cell.  The forces of the occupied slots
+// are zeroed for the step here (nothing reads the others): a memset of the whole blocks wrote
+// every spare slot, nine times the particles' on a slab in its vapour.
+template <int G>
 __global__ void __launch_bounds__(256) rebin_gather(ResidentCells RC, const Mover* __restrict__ movers,
                                                     const int* __restrict__ nstay, const int* __restrict__ nmove,
                                                     float4* __restrict__ xq_out, float4* __restrict__ v_out,
                                                     int* __restrict__ pid_out, int* __restrict__ count,
-                                                    unsigned long long* status, int* __restrict__ slot_of) {
+                                                    unsigned long long* status, int* __restrict__ slot_of,
+                                                    unsigned long long* __restrict__ force) {
     constexpr unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (c >= RC.ncells || *(volatile unsigned long long*)status != 0) return;
+    constexpr int D = (27 + G - 1) / G;
+    const int gl = threadIdx.x & (G - 1);
+    const int c = group_cell<G>();
+    if (*(volatile unsigned long long*)status != 0) return;
+    const bool cell = c < RC.ncells;
     const size_t base = (size_t)c * RC.capc;
-    int off = nstay[c];
-    bool over = false;
-    // lane d (< 27) looks up the neighbour a particle moving by direction d comes from and
-    // whether it has leavers; only those directions are walked, in order
-    int my_src = 0, my_nm = 0;
-    if (lane < 27 && lane != 13) {
-        my_src = RC.nbr[(size_t)c * 27 + (26 - lane)];
-        my_nm = nmove[my_src];
-    }
-    // The candidates of all those directions as one list, direction-major: lane d's movers
-    // occupy [pre_d, pre_d + nm_d).  Each pass loads 32 of them at once (one load latency
-    // for many directions instead of one per direction) and keeps those that moved by d.
-    int incl = my_nm;
+    int src[D], nm[D], mine = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(FULL, incl, o);
-        if (lane >= o) incl += t;
+    for (int q = 0; q < D; ++q) {
+        const int d = D * gl + q;
+        src[q] = nm[q] = 0;
+        if (cell && d < 27 && d != 13) src[q] = RC.nbr[(size_t)c * 27 + (26 - d)];
     }
-    const int my_pre = incl - my_nm;
-    const int total = __shfl_sync(FULL, incl, 31);
-    for (int t0 = 0; t0 < total; t0 += 32) {
-        const int t = t0 + lane;
-        // the direction holding candidate t: the last lane whose list starts at or before t
-        int d = 0;
 #pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
-            const int pre = __shfl_sync(FULL, my_pre, d + step);
-            if (pre <= t) d += step;
-        }
-        const int src = __shfl_sync(FULL, my_src, d);
-        const int m = t - __shfl_sync(FULL, my_pre, d);
-        Mover mv;
-        bool match = false;
-        if (t < total) {
-            mv = movers[(size_t)src * RC.mcap + m];
-            match = __float_as_int(mv.v.w) == d;
-        }
-        const unsigned bmatch = __ballot_sync(FULL, match);
-        if (match) {
-            const int o = off + __popc(bmatch & ((1u << lane) - 1u));
-            if (o < RC.capc) {
-                xq_out[base + o] = mv.x;
-                v_out[base + o] = make_float4(mv.v.x, mv.v.y, mv.v.z, 0.f);
-                pid_out[base + o] = mv.pid;
-            } else {
-                over = true;
+    for (int q = 0; q < D; ++q) {
+        const int d = D * gl + q;
+        if (cell && d < 27 && d != 13) nm[q] = nmove[src[q]];
+    }
+    const int stays = cell ? nstay[c] : 0;
+#pragma unroll
+    for (int q = 0; q < D; ++q)
+        for (int m = 0; m < nm[q]; ++m)
+            mine += __float_as_int(movers[(size_t)src[q] * RC.mcap + m].v.w) == D * gl + q;
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < G; o <<= 1) {
+        const int t = __shfl_up_sync(FULL, incl, o, G);
+        if (gl >= o) incl += t;
+    }
+    const int total = stays + __shfl_sync(FULL, incl, G - 1, G);
+    int o = stays + incl - mine;
+    if (mine > 0) {
+#pragma unroll
+        for (int q = 0; q < D; ++q)
+            for (int m = 0; m < nm[q]; ++m) {
+                const Mover mv = movers[(size_t)src[q] * RC.mcap + m];
+                if (__float_as_int(mv.v.w) != D * gl + q) continue;
+                if (o < RC.capc) {
+                    xq_out[base + o] = mv.x;
+                    v_out[base + o] = make_float4(mv.v.x, mv.v.y, mv.v.z, 0.f);
+                    pid_out[base + o] = mv.pid;
+                }
+                ++o;
             }
-        }
-        off += __popc(bmatch);
     }
-    if (__any_sync(FULL, over) && lane == 0) atomicOr(status, (unsigned long long)kStatusResidentOverflow);
-    const int n = min(off, RC.capc);
-    if (lane == 0) count[c] = n;
+    __syncwarp();                      // the group's arrivals are written
+    if (!cell) return;
+    if (gl == 0 && total > RC.capc) atomicOr(status, (unsigned long long)kStatusResidentOverflow);
+    const int n = min(total, RC.capc);
+    if (gl == 0) count[c] = n;
+    for (int k = gl; k < 3 * n; k += G) force[3 * base + k] = 0ull;
     if (slot_of != nullptr) {          // rigid systems: the slot of every particle id in this cell
-        __syncwarp();
-        for (int k = lane; k < n; k += 32) slot_of[pid_out[base + k]] = (int)(base + k);
+        for (int k = gl; k < n; k += G) slot_of[pid_out[base + k]] = (int)(base + k);
     }
 }
 
@@ -268,11 +283,12 @@ __global__ void verlet_decide(int* __restrict__ vw, float skin, float cutoff,
 // Symplectic Euler update of every particle (engine_advance, src/engine.c:1975-1979), with
 // the float expressions the host integrator evaluates: w = (float)(dt * 1/m),
 // v += f*w, x += dt*v; forces from the fixed-point accumulators of the sweep.  One thread
-// per slot (grid: ncells * capc threads).
+// per slot (grid: ncells * capc threads; G = 0), or G lanes per cell.
 //
 // With sd_gamma > 0 the update is a steepest-descent move instead (an energy minimiser for
 // unrelaxed starts; no counterpart in the reference's step): x += g f with g = sd_gamma,
 // held so that no particle moves farther than sd_dmax, and v = 0.
+template <int G>
 __global__ void __launch_bounds__(256) integrate_cells(ResidentCells RC, const int* __restrict__ count,
                                                        const unsigned long long* __restrict__ force,
                                                        const int* __restrict__ cell_engine,
@@ -288,14 +304,24 @@ __global__ void __launch_bounds__(256) integrate_cells(ResidentCells RC, const i
         done[0] += 1ull;
         done[1] += acc[kAccPairs];
     }
-    // one thread per slot of every block (the slots past a cell's count do nothing)
-    const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= (size_t)RC.ncells * RC.capc) return;
-    const int c = (int)(s / (unsigned)RC.capc);
-    if ((int)(s - (size_t)c * RC.capc) >= min(count[c], RC.capc)) return;
+    int c, k, n;
+    if constexpr (G == 0) {            // one thread per slot (those past a cell's count do nothing)
+        const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+        if (s >= (size_t)RC.ncells * RC.capc) return;
+        c = (int)(s / (unsigned)RC.capc);
+        k = (int)(s - (size_t)c * RC.capc);
+        n = min(min(count[c], RC.capc), k + 1);
+    } else {
+        c = group_cell<(G ? G : 1)>();
+        if (c >= RC.ncells) return;
+        k = threadIdx.x & (G - 1);
+        n = min(count[c], RC.capc);
+    }
+    if (k >= n) return;
     const int k_eng = cell_engine[c];
     const float dt = engine_dt[k_eng];
-    {
+    for (; k < n; k += (G ? G : 1)) {
+        const size_t s = (size_t)c * RC.capc + k;
         float4 x = xq[s], vv = v[s];
         const int type = __float_as_int(x.w);
         const float w = (float)((double)dt * engine_imass[(size_t)k_eng * max_type + type]);
@@ -311,7 +337,7 @@ __global__ void __launch_bounds__(256) integrate_cells(ResidentCells RC, const i
             xq[s] = x;
             v[s] = make_float4(0.f, 0.f, 0.f, vv.w);
             if (!isfinite(x.x + x.y + x.z)) atomicOr(status, (unsigned long long)kStatusNonFinite);
-            return;
+            continue;
         }
         vv.x = __fadd_rn(vv.x, __fmul_rn(fx, w));
         vv.y = __fadd_rn(vv.y, __fmul_rn(fy, w));

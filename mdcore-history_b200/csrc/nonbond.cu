@@ -836,7 +836,8 @@ int issue_kernels(NbState* st, const DevView& V, bool span = true) {
         const int rc = record_event(st, st->ev0);
         if (rc < 0) return rc;
     }
-    CU(cudaMemsetAsync(V.force, 0, sizeof(unsigned long long) * 3 * V.slots, st->stream));
+    if (!V.resident)                  // resident steps: zeroed with the re-binning
+        CU(cudaMemsetAsync(V.force, 0, sizeof(unsigned long long) * 3 * V.slots, st->stream));
     CU(cudaMemsetAsync(st->d_acc, 0, sizeof(unsigned long long) * kAccCount, st->stream));
     CU(cudaMemsetAsync(st->d_cell_epot, 0, sizeof(unsigned long long) * 2 * st->ncells, st->stream));
     const int cap = V.cap4;
@@ -1823,6 +1824,9 @@ ResidentCells res_cells(const NbState* st) {
 constexpr int kCellWarps = 2;
 constexpr int kCellThreads = 32 * kCellWarps;
 int res_grid(const NbState* st) { return (st->ncells + kCellWarps - 1) / kCellWarps; }
+// 8 lanes per cell instead: systems of many cells (more warps than the GPU holds at once, 148 x
+// 64, with a warp each) that hold no more particles than one warp takes.
+bool small_cells(const NbState* st) { return st->ncells >= 16384 && st->res_nparts <= 32LL * st->ncells; }
 
 // The engines' bonds for the device: global ids, the bond table of the two particles' types
 // (bonds whose types have none are dropped, as bond_eval skips them), the engine; the
@@ -2186,14 +2190,27 @@ int res_issue_step(NbState* st) {
     if (rc < 0) return rc;
     const ResidentCells RC = res_cells(st);
     const int grid = res_grid(st);
-    rebin_split<<<grid, kCellThreads, 0, st->stream>>>(RC, st->r_xq[r], st->r_v[r], st->r_pid[r], st->r_cnt[r], st->r_xq[o],
-                                              st->r_v[o], st->r_pid[o], st->r_nstay, st->r_nmove, st->r_movers,
-                                              st->r_status, st->verlet ? st->r_vw : nullptr);
     bool rigid = false;
     for (struct engine* e : st->engines) rigid = rigid || e->nr_rigids > 0;
-    rebin_gather<<<grid, kCellThreads, 0, st->stream>>>(RC, st->r_movers, st->r_nstay, st->r_nmove, st->r_xq[o], st->r_v[o],
-                                               st->r_pid[o], st->r_cnt[o], st->r_status,
-                                               (rigid || res_bonded(st)) ? st->r_slot_of : nullptr);
+    const bool small = small_cells(st);
+    const int sgrid = (int)(((size_t)st->ncells * 8 + 255) / 256);
+    int* slot_of = (rigid || res_bonded(st)) ? st->r_slot_of : nullptr;
+    const int* rebuild = st->verlet ? st->r_vw : nullptr;
+    if (small) {
+        rebin_split<8><<<sgrid, 256, 0, st->stream>>>(RC, st->r_xq[r], st->r_v[r], st->r_pid[r], st->r_cnt[r],
+                                                      st->r_xq[o], st->r_v[o], st->r_pid[o], st->r_nstay, st->r_nmove,
+                                                      st->r_movers, st->r_status, rebuild);
+        rebin_gather<8><<<sgrid, 256, 0, st->stream>>>(RC, st->r_movers, st->r_nstay, st->r_nmove, st->r_xq[o],
+                                                       st->r_v[o], st->r_pid[o], st->r_cnt[o], st->r_status, slot_of,
+                                                       st->r_force);
+    } else {
+        rebin_split<32><<<grid, kCellThreads, 0, st->stream>>>(RC, st->r_xq[r], st->r_v[r], st->r_pid[r], st->r_cnt[r],
+                                                               st->r_xq[o], st->r_v[o], st->r_pid[o], st->r_nstay,
+                                                               st->r_nmove, st->r_movers, st->r_status, rebuild);
+        rebin_gather<32><<<grid, kCellThreads, 0, st->stream>>>(RC, st->r_movers, st->r_nstay, st->r_nmove, st->r_xq[o],
+                                                                st->r_v[o], st->r_pid[o], st->r_cnt[o], st->r_status,
+                                                                slot_of, st->r_force);
+    }
     CU(cudaGetLastError());
     const unsigned vblocks = (unsigned)(((size_t)st->ncells * st->capc + 255) / 256);
     if (st->verlet) {
@@ -2259,10 +2276,10 @@ int res_issue_step(NbState* st) {
     }
     if (!fuse) {
         const unsigned slot_blocks = (unsigned)(((size_t)st->ncells * st->capc + 255) / 256);
-        integrate_cells<<<slot_blocks, 256, 0, st->stream>>>(RC, st->r_cnt[o], st->r_force, st->r_cell_engine,
-                                                             st->r_engine_dt, st->r_engine_imass, st->max_type,
-                                                             st->r_xq[o], st->r_v[o], st->r_status, st->d_acc,
-                                                             st->r_done, st->sd_gamma, st->sd_dmax);
+        auto update = small ? integrate_cells<8> : integrate_cells<0>;
+        update<<<small ? (unsigned)sgrid : slot_blocks, 256, 0, st->stream>>>(
+            RC, st->r_cnt[o], st->r_force, st->r_cell_engine, st->r_engine_dt, st->r_engine_imass, st->max_type, st->r_xq[o],
+            st->r_v[o], st->r_status, st->d_acc, st->r_done, st->sd_gamma, st->sd_dmax);
         CU(cudaGetLastError());
     }
     for (size_t k = 0; k < st->engines.size(); k++) {
