@@ -633,7 +633,8 @@ def measure(workload, args, rank, world, local_rank, dist, with_cpu):
             # kernels of one resident step: re-binning (2), sort, queue compaction (3, systems
             # with empty cells), sweep, integration, constraints (rigid, one per engine)
             # (the update runs inside the constraint kernel when every particle of a single
-            # system is in a rigid group)
+            # system is in a rigid group); the cell form, when the autotuner keeps it, launches one
+            # more (its unit list, sweep and candidate count for sort and sweep), not counted here
             fused = (rigid and len(systems) == 1 and
                      len(set(np.asarray(systems[0].rigid)[:, :2].astype(int).ravel().tolist())) == systems[0].n)
             per_step = 2 + 1 + 3 * int(compact) + 1 + int(not fused) + int(rigid) * len(engines)
