@@ -1375,6 +1375,19 @@ int load_state(NbState* st) {
     CU(cudaMemcpy(st->d_emask, emask.data(), nid * sizeof(unsigned), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(st->d_exoff, cnt.data(), (nid + 1) * sizeof(int), cudaMemcpyHostToDevice));
     CU(cudaMemcpy(st->d_exlist, exlist.data(), exlist.size() * sizeof(int), cudaMemcpyHostToDevice));
+    // Engines that evaluate in the cell form from the start have its lists before their first
+    // evaluation, like everything above.
+    if (use_cells(st, false)) {
+        size_t slots = 4;
+        int most = 0;
+        for (const struct cell* c : st->flat_cells) {
+            slots += (size_t)((c->count + 3) & ~3);
+            most = std::max(most, c->count);
+        }
+        int rc = build_cell_tasks(st);
+        if (rc == 0) rc = reserve_units(st, slots, (std::min(most, kMaxPartsPerCell) + 3) & ~3);
+        if (rc < 0) return rc;
+    }
     return 0;
 }
 
