@@ -429,7 +429,10 @@ def roofline_obj(M, local_rank, pairs, sweep_ms, layout, workload):
     peak = M.fp32_peak_tflops(local_rank)
     achieved = FLOPS_PER_PAIR * pairs / (sweep_ms * 1e-3) / 1e12
     return {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-            "traffic": read_traffic(workload), "kernel": "sweep_tiled" if layout else "sweep_tuned",
+            "traffic": read_traffic(workload),      # of the queue form's sweep
+            # one table: the autotuner may keep the cell form (sweep_cells) instead
+            "kernel": ("sweep_tiled" if layout else "sweep_tuned")
+                      + (" or sweep_cells, the faster" if workload in ("replicas", "argon") else ""),
             "kernel_ms": sweep_ms, "flops_per_pair": FLOPS_PER_PAIR,
             "peak_source": "measured FP32 FMA loop on this GPU (engine_cuda_fp32_peak); "
                            "MEASURED_PEAKS.json has no FP32 figure"}

@@ -28,8 +28,8 @@
 // slots 60 % busy with 2.75 warps per scheduler (the accumulators limit an SM to 12 or 13
 // warps), shared-memory pipe 50 %, DRAM idle; 0.86 ms per sweep against 1.19 and no sort (0.13);
 // a resident step 1.47 -> 0.94 ms.  About half of the instructions evaluate pairs (two per lane
-// and iteration, 52 % of the lane slots carrying one: the lists by number of rows give that,
-// one list gives 40 %), a quarter tests rows.  Solvated chains, 12,400 atoms, tables in global
+// and iteration, 52 % of the lane slots carrying one, counted on the CPU: the two lists by
+// number of rows give that, one list gives 40 %), a quarter tests rows.  Solvated chains, 12,400 atoms, tables in global
 // memory, charges: sweep 0.55 -> 0.27 ms.  On cells of 135 particles (water) it loses, 0.45
 // against 0.28 ms per step: every strip walks the whole neighbourhood again.
 // The tables are held in 8 interleaved copies, one per lane of a quarter warp, so that the
@@ -46,8 +46,9 @@ constexpr int kCellRing = 64;            // near list
 constexpr int kCellList = 96;            // evaluation lists: up to 31 left of each class and 32 new
 
 // One worker warp's slice of shared memory; ROWS (24 or 32): i particles of a unit at most.
-// The accumulators are most of it: 24 rows leave room for 13 warps instead of 11, 32 need fewer
-// units for cells of 25 to 32 particles.
+// The accumulators are most of it: 24 rows leave room for 13 warps instead of 12, 32 need fewer
+// units for cells of 25 to 32 particles (resident steps with 24 / 32 rows: slab 0.92 / 0.99 ms,
+// replicas 1.04 / 0.94; the autotuner times both).
 template <int ROWS>
 struct CellWarp {
     float acc[3][ROWS][32];         // i force by component, row, lane
