@@ -506,8 +506,9 @@ int engine_getforces(struct engine *e, double *f, int N);
 int engine_getcells(struct engine *e, int *cell, int N);
 /* Counters and FP64 sums of the last nonbonded evaluation. */
 int engine_nonbond_stats(struct engine *e, struct nb_stats *out);
-/* The sorted key lists the device built in the last evaluation for cell cid
- * (13 x count entries, sid-major, same key format as src/runner_dosort.c:148-149). */
+/* The sorted key lists of cell cid in the last host-buffer evaluation (resident steps leave
+ * them alone; after an evaluation in the cell form, which sorts nothing, they are built here):
+ * 13 x count entries, sid-major, same key format as src/runner_dosort.c:148-149. */
 int engine_cuda_getsort(struct engine *e, int cid, unsigned int *keys, int size);
 /* Device-resident force evaluation: positions already on the device (uploaded by
  * engine_cuda_load_parts), forces left on the device.  Used to time the kernels alone. */

@@ -96,7 +96,9 @@ struct NbState {
     int2* d_units = nullptr;       // units of the evaluation, their number and the queue head
     size_t units_cap = 0;
     int* d_unit_words = nullptr;   // queue head, units, count candidates (resident steps), 1
-    bool keys_stale = true;        // the host-path / resident sort keys are not the last evaluation's
+    // The sort keys of a buffer (d_keys, r_keys) are not its last evaluation's: none has been
+    // sorted there yet, or the last one ran in the cell form.
+    bool host_keys_stale = true, res_keys_stale = true;
     int fp32acc = 0;               // plain form: forces accumulated in FP32 (float atomics)
     float* d_force32 = nullptr;    // float forces of FP32 accumulation (3 per slot)
     size_t force32_slots = 0;
@@ -314,6 +316,7 @@ int alloc_particles(NbState* st, int ncap) {
     cudaFreeHost(st->h_xq); cudaFreeHost(st->h_pid); cudaFreeHost(st->h_force);
     st->h_xq = nullptr; st->h_pid = nullptr; st->h_force = nullptr;
     ++st->buf_gen;
+    st->host_keys_stale = true;
     if (dev_alloc(&st->d_xq, ncap) || dev_alloc(&st->d_pid, ncap) || dev_alloc(&st->d_keys, 13 * (size_t)ncap) ||
         dev_alloc(&st->d_force, 3 * (size_t)ncap))
         return engine_err_cuda;
@@ -848,7 +851,6 @@ int issue_kernels(NbState* st, const DevView& V, bool span = true) {
         return rc;
     }
     const bool cells = use_cells(st, V.resident || st->stepping);
-    st->keys_stale = cells;
     if (!cells) {
         const int rc0 = launch_sort(V.xq, V.cstart, V.ccount, st->d_cmask, V.keys, st->d_cscale, st->ncells, V.cpc, cap,
                                     st->d_acc, V.abort, st->capturing, st->stream, V.rebuild);
@@ -858,6 +860,7 @@ int issue_kernels(NbState* st, const DevView& V, bool span = true) {
         if (rc0 == 0) rc0 = reserve_units(st, V.slots, cap);
         if (rc0 < 0) return rc0;
     }
+    if (!st->capturing) (V.resident ? st->res_keys_stale : st->host_keys_stale) = cells;
 
     Params P;
     P.xq = V.xq;
@@ -932,16 +935,16 @@ int issue_kernels(NbState* st, const DevView& V, bool span = true) {
 
 int issue_kernels(NbState* st) { return issue_kernels(st, host_view(st)); }
 
-// The sort keys of the uploaded particles, for readers of the keys after evaluations in the
-// cell form, which needs none.
-int sort_keys(NbState* st, const DevView& V) {
-    if (V.cap4 == 0) return 0;
+// The sort keys of a view's particles, for readers of the keys when its buffer's are stale (the
+// cell form sorts nothing).
+int sort_stale_keys(NbState* st, const DevView& V) {
+    bool& stale = V.resident ? st->res_keys_stale : st->host_keys_stale;
+    if (!stale || V.cap4 == 0) return 0;
     const int rc = launch_sort(V.xq, V.cstart, V.ccount, st->d_cmask, V.keys, st->d_cscale, st->ncells, V.cpc, V.cap4,
                                st->d_acc, nullptr, false, st->stream);
-    if (rc == 0) st->keys_stale = false;
+    if (rc == 0) stale = false;
     return rc;
 }
-int sort_host_keys(NbState* st) { return sort_keys(st, host_view(st)); }
 
 void drop_graph(NbState* st) {
     if (st->graph_exec) cudaGraphExecDestroy(st->graph_exec);
@@ -976,7 +979,7 @@ int launch_kernels(NbState* st) {
     const long long key = launch_key(st);
     if (st->graph_exec != nullptr && st->graph_key == key) {
         CU(cudaGraphLaunch(st->graph_exec, st->stream));
-        st->keys_stale = use_cells(st, st->stepping);
+        st->host_keys_stale = use_cells(st, st->stepping);
         return 0;
     }
     if (st->prepared_key != key) {
@@ -1000,6 +1003,7 @@ int launch_kernels(NbState* st) {
     CU(cudaGraphInstantiate(&st->graph_exec, g, 0));
     st->graph_key = key;
     CU(cudaGraphLaunch(st->graph_exec, st->stream));
+    st->host_keys_stale = use_cells(st, st->stepping);
     return 0;
 }
 
@@ -1991,6 +1995,7 @@ int res_alloc(NbState* st, int capc, int mcap, long long n) {
         CU(cudaMemset(st->r_pid[q], 0, sizeof(int) * slots));
     }
     CU(cudaMalloc(&st->r_keys, sizeof(unsigned) * 13 * slots));
+    st->res_keys_stale = true;
     CU(cudaMalloc(&st->r_force, sizeof(unsigned long long) * 3 * slots));
     CU(cudaMemset(st->r_force, 0, sizeof(unsigned long long) * 3 * slots));
     CU(cudaMalloc(&st->r_cnt[0], sizeof(int) * (nc + 1)));
@@ -2379,7 +2384,7 @@ int res_issue_steps(NbState* st, int nsteps) {
             if (rc < 0) return rc;
         } else if (st->rgraph_exec[side] != nullptr && st->rgraph_key[side] == key) {
             CU(cudaGraphLaunch(st->rgraph_exec[side], st->stream));
-            st->keys_stale = use_cells(st, true);
+            st->res_keys_stale = use_cells(st, true);
         } else if (st->rprepared[side] != key) {
             const int rc = res_issue_step(st);
             if (rc < 0) return rc;
@@ -2404,6 +2409,7 @@ int res_issue_steps(NbState* st, int nsteps) {
             CU(cudaGraphInstantiate(&st->rgraph_exec[side], g, 0));
             st->rgraph_key[side] = key;
             CU(cudaGraphLaunch(st->rgraph_exec[side], st->stream));
+            st->res_keys_stale = use_cells(st, true);
         }
         st->rside = 1 - side;
     }
@@ -3235,8 +3241,8 @@ extern "C" int engine_cuda_getsort(struct engine* e, int cid, unsigned int* keys
     if (size < 13 * n) return engine_err_range;
     std::vector<unsigned> buf(13 * (size_t)pad + 1);
     CU(cudaSetDevice(st->device));
-    if (st->keys_stale && !st->res_active && st->resident_valid) {      // the cell form sorts nothing
-        const int rc = sort_host_keys(st);
+    if (st->resident_valid) {          // the uploaded particles', also during resident steps
+        const int rc = sort_stale_keys(st, host_view(st));
         if (rc < 0) return rc;
     }
     CU(cudaStreamSynchronize(st->stream));
@@ -3909,7 +3915,7 @@ extern "C" int engine_sched_features(struct engine* e, float* features_out, int 
     const int* cstart = res ? st->r_cstart : st->d_cstart;
     const int* ccount = res ? st->r_cnt[st->rside] : st->d_ccount;
     const unsigned* keys = res ? st->r_keys : st->d_keys;
-    if (st->keys_stale && (res || st->resident_valid)) {
+    if (res || st->resident_valid) {
         DevView V;
         if (res) {
             V.xq = xq;
@@ -3918,10 +3924,11 @@ extern "C" int engine_sched_features(struct engine* e, float* features_out, int 
             V.ccount = ccount;
             V.cap4 = st->capc;
             V.cpc = st->res_nparts <= 32LL * st->ncells ? kSortWarps : 1;
+            V.resident = true;
         } else {
             V = host_view(st);
         }
-        const int rc = sort_keys(st, V);
+        const int rc = sort_stale_keys(st, V);
         if (rc < 0) return rc;
     }
     cell_type0<<<(st->ncells + 255) / 256, 256, 0, st->stream>>>(xq, cstart, ccount, st->ncells, ss->d_ctype0);

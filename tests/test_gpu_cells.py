@@ -149,3 +149,36 @@ def test_steps_of_several_tables_keep_the_queue_form(monkeypatch):
         e.close()
     for other in out[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(out[0][:2], other[:2]))
+
+
+def chain_mix():
+    """Many tables, no bonds: force evaluations run the cell form by default, steps the queue form."""
+    s = W.chains_water(nchains=6, length=20, nwater=200, box=(4.0, 4.0, 4.0), seed=2, angles_dihedrals=False)
+    s.bonds = None
+    return s
+
+
+@pytest.mark.parametrize("graph", [False, True])
+@pytest.mark.parametrize("calls", ["step, nonbond", "nonbond, resident steps", "nonbond, resident steps, end",
+                                   "resident steps, nonbond, end"])
+def test_keys_of_mixed_calls_are_the_queue_forms(calls, graph, monkeypatch):
+    """Host evaluations and resident steps have sort keys of their own; an engine whose evaluations
+    run the cell form and whose steps run the queue form answers as one of the queue form only."""
+    out = []
+    for form in (None, "queue"):
+        if form:
+            monkeypatch.setenv("MDB_SWEEP_FORM", form)
+        e = M.Engine.from_system(chain_mix())
+        e.graph(graph)
+        for call in calls.split(", "):
+            if call == "resident steps":
+                e.resident_begin()
+                e.resident_steps(5)
+            else:
+                for _ in range(1 if call == "end" else 4):
+                    {"step": e.step, "nonbond": e.nonbond, "end": e.resident_end}[call]()
+        counts = np.bincount(e.cells(), minlength=8)
+        keys = [] if "end" in calls else [e.sortkeys(c, int(counts[c])) for c in range(8)]
+        out.append(keys + [e.sched_features()])
+        e.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
