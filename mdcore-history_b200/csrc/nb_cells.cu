@@ -309,7 +309,7 @@ __device__ __forceinline__ void cell_window(const Params& P, CellWarp<ROWS>& W, 
             eB = okB ? eB : 0.f;
             fB = okB ? fB : 0.f;
         }
-        const f32x2 f = pack2(-fA, -fB);         // 0 for a rejected pair; displacements are finite
+        const f32x2 f = pack2(-fA, -fB);         // 0 for a rejected pair; positions are finite
         const f32x2 wx = mul2(f, dx), wy = mul2(f, dy), wz = mul2(f, dz);
         fx = add2(fx, wx);
         fy = add2(fy, wy);
@@ -551,7 +551,16 @@ __global__ void __launch_bounds__(kCellWarps * 32 + 32, 1) sweep_cells(CellParam
         // the rows
         float4 xi = make_float4(0.f, 0.f, 0.f, 0.f);
         if (lane < nr) xi = P.xq[start + r0 + lane];
-        const float ni = lane < nr ? fmaf(xi.z, xi.z, fmaf(xi.y, xi.y, xi.x * xi.x)) : INFINITY;
+        float ni = lane < nr ? fmaf(xi.z, xi.z, fmaf(xi.y, xi.y, xi.x * xi.x)) : INFINITY;
+        // A non-finite position (or one whose square overflows: beyond 1e19 nm) has no pairs: such
+        // a row is treated as those past the last (no test passes it, and its position in W is
+        // finite, since rejected pairs multiply their displacement by 0), such a j is dropped by
+        // the box test.
+        const bool in = ni < INFINITY;
+        if (!in) {
+            xi.x = xi.y = xi.z = 0.f;
+            ni = INFINITY;
+        }
         W.rx[lane] = xi.x;
         W.ry[lane] = xi.y;
         W.rz[lane] = xi.z;
@@ -568,7 +577,6 @@ __global__ void __launch_bounds__(kCellWarps * 32 + 32, 1) sweep_cells(CellParam
             rt[4] = -2.f * xi.z;
             rt[6] = ni;
         }
-        const bool in = lane < nr;
         const float lox = warp_min(in ? xi.x : INFINITY), hix = warp_max(in ? xi.x : -INFINITY);
         const float loy = warp_min(in ? xi.y : INFINITY), hiy = warp_max(in ? xi.y : -INFINITY);
         const float loz = warp_min(in ? xi.z : INFINITY), hiz = warp_max(in ? xi.z : -INFINITY);
@@ -621,8 +629,7 @@ __global__ void __launch_bounds__(kCellWarps * 32 + 32, 1) sweep_cells(CellParam
                 const ulonglong2 p = *reinterpret_cast<const ulonglong2*>(&W.rt[k]);
                 const ulonglong2 s = *reinterpret_cast<const ulonglong2*>(&W.rt[k + 1]);
                 const f32x2 d = add2(fma2(p.x, x2, fma2(p.y, y2, fma2(s.x, z2, s.y))), n2);
-                // r^2 - cutoff^2: negative when near (not for an infinite or NaN position, which
-                // the exact test would reject)
+                // r^2 - cutoff^2: negative when near
                 float dA, dB;
                 unpack2(d, dA, dB);
                 near = __funnelshift_l(__float_as_uint(dA), near, 1);
@@ -673,7 +680,8 @@ __global__ void __launch_bounds__(kCellWarps * 32 + 32, 1) sweep_cells(CellParam
                 const float gx = fmaxf(fmaxf(lox - x, x - hix), 0.f), gy = fmaxf(fmaxf(loy - y, y - hiy), 0.f),
                             gz = fmaxf(fmaxf(loz - z, z - hiz), 0.f);
                 const float nj = fmaf(z, z, fmaf(y, y, x * x));
-                const bool far = fmaf(gz, gz, fmaf(gy, gy, gx * gx)) > fmaf(kSlack, nj + nimax, sh.w);
+                const bool far = !(nj < INFINITY) ||
+                                 fmaf(gz, gz, fmaf(gy, gy, gx * gx)) > fmaf(kSlack, nj + nimax, sh.w);
                 const unsigned ball = __ballot_sync(FULL, on && !far);
                 if (on && !far) {
                     const int o = (b0 + nb + __popc(ball & ((1u << lane) - 1u))) & (kCellRing - 1);

@@ -5,6 +5,8 @@ exact, energy, virial and forces within the parity bounds of the oracle, at the 
 its strips, lists and masks end (cells of 0 to 90 particles, a cell of 1,000, a vapour, list
 and mask exclusions, many tables), and the same results alone, in a batch,
 resident and through engine_step."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -182,3 +184,42 @@ def test_keys_of_mixed_calls_are_the_queue_forms(calls, graph, monkeypatch):
         out.append(keys + [e.sched_features()])
         e.close()
     assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+def positions(e):
+    """The engine's own cell-relative position (3 floats) of every particle by id."""
+    partlist = C.c_void_p.from_address(e.ptr.value + 8 + 168).value     # struct space, after its flags
+    out = []
+    for i, p in enumerate((C.c_void_p * e.n).from_address(partlist)):
+        assert C.c_int.from_address(p + 52).value == i                  # struct part: id
+        out.append(np.frombuffer((C.c_float * 3).from_address(p), np.float32))
+    return out
+
+
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan, 1e12])
+@pytest.mark.parametrize("name", ["far-exclusions", "water", "chains"])
+def test_non_finite_positions_have_no_pairs(name, bad, monkeypatch):
+    """Particles at every place of a cell's list lost to infinity, or far away and from each other:
+    no pairs and no force of their own, the others' forces those of the queue form."""
+    sysm = SYSTEMS[name]()
+    out = {}
+    for form in ("queue", "cells", "cells24"):
+        monkeypatch.setenv("MDB_SWEEP_FORM", form)
+        e = M.Engine.from_system(sysm)
+        x = positions(e)
+        c = e.cells()
+        lost = [np.flatnonzero(c == k)[k % 24] for k in range(c.max() + 1) if (c == k).sum() > k % 24]
+        lost += [i for k in range(0, c.max() + 1, 3) for i in np.flatnonzero(c == k)[:1]]
+        for k, i in enumerate(lost):
+            x[i][k % 3] = bad * (k + 1)
+        e.nonbond()
+        st = e.stats()
+        out[form] = e.forces(), (st.status, st.pairs, st.excluded, st.candidates), st.epot
+        e.close()
+    f0, counts, epot = out["queue"]
+    assert counts[0] == 0 and counts[1] > 1000 and not f0[lost].any()
+    for form in ("cells", "cells24"):
+        f, n, ep = out[form]
+        assert n == counts and abs(ep - epot) <= 2e-6 * abs(epot)
+        err = force_errors(f, f0)          # each form within the parity bounds (2e-6, 2e-5) of the exact forces
+        assert err["global_rel"] <= 4e-6 and err["max_over_frms"] <= 4e-5, err
