@@ -653,6 +653,18 @@ int engine_cuda_setlayout(struct engine *e, int layout, int stages, int occupanc
 int engine_cuda_autotune(struct engine *e, int reps, int *warps, int *layout, int *stages, int *occupancy,
                          float *ms);
 
+/* How the last evaluation on the device ran (a host-buffer evaluation or resident step of this
+ * engine; of a grouped batch step, its first group's): form, the i particles of a unit of the
+ * cell form at most (24 or 32, else 0), and whether its launches went out as a CUDA graph.  Any
+ * pointer may be NULL. */
+enum {
+    engine_cuda_form_none = 0,   /* no evaluation yet */
+    engine_cuda_form_plain,      /* one block per task (engine_cuda_settune) */
+    engine_cuda_form_queue,      /* persistent sweep over the task queue */
+    engine_cuda_form_cells       /* cell form */
+};
+int engine_cuda_getform(struct engine *e, int *form, int *rows, int *graph);
+
 /* ---- device-resident time steps (replace engine_step, src/engine.c:2070-2240, while
  * the particles stay on the device) ----
  * engine_cuda_resident_begin uploads every particle into fixed blocks of slots per cell
@@ -758,6 +770,7 @@ int engine_batch_settune(struct engine_batch *b, int warps, int plain);
 int engine_batch_graph(struct engine_batch *b, int enable);
 int engine_batch_autotune(struct engine_batch *b, int reps, int *warps, int *layout, int *stages, int *occupancy,
                           float *ms);
+int engine_batch_getform(struct engine_batch *b, int *form, int *rows, int *graph);
 int engine_batch_setlayout(struct engine_batch *b, int layout, int stages, int occupancy);
 int engine_batch_ntasks(struct engine_batch *b);
 /* Device-resident steps of every engine of the batch (engine_cuda_resident_*): one

@@ -99,6 +99,8 @@ struct NbState {
     // The sort keys of a buffer (d_keys, r_keys) are not its last evaluation's: none has been
     // sorted there yet, or the last one ran in the cell form.
     bool host_keys_stale = true, res_keys_stale = true;
+    // How the last evaluation ran (engine_cuda_getform).
+    int last_form = engine_cuda_form_none, last_rows = 0, last_graph = 0;
     int fp32acc = 0;               // plain form: forces accumulated in FP32 (float atomics)
     float* d_force32 = nullptr;    // float forces of FP32 accumulation (3 per slot)
     size_t force32_slots = 0;
@@ -831,6 +833,16 @@ DevView host_view(const NbState* st) {
     return V;
 }
 
+// Bookkeeping of an evaluation being issued directly or as a graph: its form, and whether the
+// sort keys of its buffer are its own (the cell form sorts nothing).  steps: of a time step.
+void note_evaluation(NbState* st, bool resident, bool steps, bool graph) {
+    const bool cells = use_cells(st, steps);
+    (resident ? st->res_keys_stale : st->host_keys_stale) = cells;
+    st->last_form = cells ? engine_cuda_form_cells : st->plain ? engine_cuda_form_plain : engine_cuda_form_queue;
+    st->last_rows = cells ? st->cell_rows : 0;
+    st->last_graph = graph;
+}
+
 // The launches of one evaluation: zero the accumulators, sort, (compact the queue,) sweep.
 // span: record ev0/ev1 around them (inside a captured graph as event nodes, so that they
 // time the device work and not the host's launch).
@@ -860,7 +872,7 @@ int issue_kernels(NbState* st, const DevView& V, bool span = true) {
         if (rc0 == 0) rc0 = reserve_units(st, V.slots, cap);
         if (rc0 < 0) return rc0;
     }
-    if (!st->capturing) (V.resident ? st->res_keys_stale : st->host_keys_stale) = cells;
+    if (!st->capturing) note_evaluation(st, V.resident, V.resident || st->stepping, false);
 
     Params P;
     P.xq = V.xq;
@@ -979,7 +991,7 @@ int launch_kernels(NbState* st) {
     const long long key = launch_key(st);
     if (st->graph_exec != nullptr && st->graph_key == key) {
         CU(cudaGraphLaunch(st->graph_exec, st->stream));
-        st->host_keys_stale = use_cells(st, st->stepping);
+        note_evaluation(st, false, st->stepping, true);
         return 0;
     }
     if (st->prepared_key != key) {
@@ -1003,7 +1015,7 @@ int launch_kernels(NbState* st) {
     CU(cudaGraphInstantiate(&st->graph_exec, g, 0));
     st->graph_key = key;
     CU(cudaGraphLaunch(st->graph_exec, st->stream));
-    st->host_keys_stale = use_cells(st, st->stepping);
+    note_evaluation(st, false, st->stepping, true);
     return 0;
 }
 
@@ -2384,7 +2396,7 @@ int res_issue_steps(NbState* st, int nsteps) {
             if (rc < 0) return rc;
         } else if (st->rgraph_exec[side] != nullptr && st->rgraph_key[side] == key) {
             CU(cudaGraphLaunch(st->rgraph_exec[side], st->stream));
-            st->res_keys_stale = use_cells(st, true);
+            note_evaluation(st, true, true, true);
         } else if (st->rprepared[side] != key) {
             const int rc = res_issue_step(st);
             if (rc < 0) return rc;
@@ -2409,7 +2421,7 @@ int res_issue_steps(NbState* st, int nsteps) {
             CU(cudaGraphInstantiate(&st->rgraph_exec[side], g, 0));
             st->rgraph_key[side] = key;
             CU(cudaGraphLaunch(st->rgraph_exec[side], st->stream));
-            st->res_keys_stale = use_cells(st, true);
+            note_evaluation(st, true, true, true);
         }
         st->rside = 1 - side;
     }
@@ -2775,6 +2787,18 @@ static int st_setlayout(NbState* st, int layout, int stages, int occupancy) {
     st->queue_form = !(st->tuned_cells && layout == st->tuned_shape[1] && stages == st->tuned_shape[2] &&
                        occupancy == st->tuned_shape[3]);
     return 0;
+}
+
+static int st_getform(const NbState* st, int* form, int* rows, int* graph) {
+    if (form) *form = st->last_form;
+    if (rows) *rows = st->last_rows;
+    if (graph) *graph = st->last_graph;
+    return 0;
+}
+
+extern "C" int engine_cuda_getform(struct engine* e, int* form, int* rows, int* graph) {
+    if (e == nullptr || e->cuda == nullptr) return engine_err_null;
+    return st_getform(state(e), form, rows, graph);
 }
 
 extern "C" int engine_cuda_setlayout(struct engine* e, int layout, int stages, int occupancy) {
@@ -3191,6 +3215,9 @@ int st_step_grouped(NbState* st, int k) {
         tot.status |= c->bstats.status;
     }
     if (err != 0) return err;
+    st->last_form = st->groups[0]->last_form;
+    st->last_rows = st->groups[0]->last_rows;
+    st->last_graph = st->groups[0]->last_graph;
     st->bstats.epot = tot.epot;
     st->bstats.virial = tot.virial;
     st->bstats.pairs = tot.pairs;
@@ -3422,6 +3449,11 @@ extern "C" int engine_batch_kernel_times(struct engine_batch* b, float* total_ms
 extern "C" int engine_batch_settune(struct engine_batch* b, int warps, int plain) {
     if (b == nullptr) return engine_err_null;
     return st_settune(bstate(b), warps, plain);
+}
+
+extern "C" int engine_batch_getform(struct engine_batch* b, int* form, int* rows, int* graph) {
+    if (b == nullptr) return engine_err_null;
+    return st_getform(bstate(b), form, rows, graph);
 }
 
 extern "C" int engine_batch_graph(struct engine_batch* b, int enable) {

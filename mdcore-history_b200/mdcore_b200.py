@@ -152,6 +152,8 @@ def lib() -> C.CDLL:
         "engine_batch_setstream": (C.c_int, [vp, vp]),
         "engine_batch_kernel_times": (C.c_int, [vp, P(C.c_float), P(C.c_float)]),
         "engine_batch_settune": (C.c_int, [vp, C.c_int, C.c_int]),
+        "engine_cuda_getform": (C.c_int, [vp, ip, ip, ip]),
+        "engine_batch_getform": (C.c_int, [vp, ip, ip, ip]),
         "engine_batch_graph": (C.c_int, [vp, C.c_int]),
         "engine_batch_autotune": (C.c_int, [vp, C.c_int, ip, ip, ip, ip, P(C.c_float)]),
         "engine_batch_ntasks": (C.c_int, [vp]),
@@ -513,6 +515,10 @@ class Engine:
                                              C.byref(ms)), "engine_cuda_autotune")
         return w.value, lay.value, stg.value, occ.value, ms.value
 
+    def form(self):
+        """Form(name, rows, graph) of the last evaluation (engine_cuda_getform)."""
+        return _form(self.lib.engine_cuda_getform, self.ptr)
+
     def ntasks(self) -> int:
         return _check(self.lib.engine_cuda_ntasks(self.ptr), "engine_cuda_ntasks")
 
@@ -640,6 +646,15 @@ def _resident_info(fn, ptr):
     return ResidentInfo(a.value, b.value, c.value, d.value, g.value)
 
 
+Form = collections.namedtuple("Form", "name rows graph")
+
+
+def _form(fn, ptr):
+    f, r, g = C.c_int(), C.c_int(), C.c_int()
+    _check(fn(ptr, C.byref(f), C.byref(r), C.byref(g)), fn.__name__)
+    return Form(("none", "plain", "queue", "cells")[f.value], r.value, bool(g.value))
+
+
 class Batch:
     """Many engines (replicas) evaluated together: one sort and one persistent sweep
     launch over all of them (engine_batch_*).  The engines need no device state of their
@@ -742,6 +757,9 @@ class Batch:
         _check(self.lib.engine_batch_autotune(self.ptr, reps, C.byref(w), C.byref(lay), C.byref(stg), C.byref(occ),
                                               C.byref(ms)), "engine_batch_autotune")
         return w.value, lay.value, stg.value, occ.value, ms.value
+
+    def form(self):
+        return _form(self.lib.engine_batch_getform, self.ptr)
 
     def ntasks(self) -> int:
         return _check(self.lib.engine_batch_ntasks(self.ptr), "engine_batch_ntasks")

@@ -78,6 +78,7 @@ def test_cell_form_vs_oracle_and_queue_form(name, cells, monkeypatch):
         monkeypatch.setenv("MDB_SWEEP_FORM", form)
         e = M.Engine.from_system(sysm)
         e.nonbond()
+        assert e.form() == (("queue", 0) if form == "queue" else ("cells", 24 if form == "cells24" else 32)) + (False,)
         out[form] = e.forces(), e.stats(), [e.sortkeys(c, int((e.cells() == c).sum())) for c in (0, 1, 5)]
         e.close()
     f, st, keys = out[cells]
@@ -102,11 +103,13 @@ def test_cell_form_is_the_same_alone_in_a_batch_and_resident(name, monkeypatch):
     b = M.Batch(engines)
     b.graph(True)
     b.resident_begin().resident_steps(7)
+    assert b.form()[:2] == ("cells", 32)
     b.resident_sync()
     for s, r in zip(systems, engines):
         e = M.Engine.from_system(s)
         for _ in range(7):
             e.step()
+        assert e.form().name == "cells"
         assert all(np.array_equal(x, y) for x, y in zip(e.parts(), r.parts()))
         assert e.energies() == r.energies()
         st = e.stats()
@@ -131,6 +134,7 @@ def test_candidates_of_the_last_step_of_every_call(monkeypatch):
             e.resident_steps(k)
             e.resident_sync()
             got[form].append((e.stats().pairs, e.stats().candidates))
+            assert e.form().name == form
         e.close()
     assert got["cells"] == got["queue"]
 
@@ -147,7 +151,10 @@ def test_steps_of_several_tables_keep_the_queue_form(monkeypatch):
         e = M.Engine.from_system(sysm)
         for _ in range(3):
             e.step_host() if host else e.step()
+            assert e.form().name == "queue"
         out.append(e.parts())
+        e.nonbond()
+        assert e.form().name == (form or "cells")
         e.close()
     for other in out[1:]:
         assert all(np.array_equal(a, b) for a, b in zip(out[0][:2], other[:2]))
@@ -213,6 +220,7 @@ def test_non_finite_positions_have_no_pairs(name, bad, monkeypatch):
         for k, i in enumerate(lost):
             x[i][k % 3] = bad * (k + 1)
         e.nonbond()
+        assert e.form().name == form[:5]
         st = e.stats()
         out[form] = e.forces(), (st.status, st.pairs, st.excluded, st.candidates), st.epot
         e.close()
@@ -223,3 +231,98 @@ def test_non_finite_positions_have_no_pairs(name, bad, monkeypatch):
         assert n == counts and abs(ep - epot) <= 2e-6 * abs(epot)
         err = force_errors(f, f0)          # each form within the parity bounds (2e-6, 2e-5) of the exact forces
         assert err["global_rel"] <= 4e-6 and err["max_over_frms"] <= 4e-5, err
+
+
+def test_autotuner_choice_and_what_undoes_it():
+    """A large system of one table is tuned to the cell form (some 20 % ahead there); the returned
+    shape stands for it, any other shape and a queue order given afterwards select the queue form."""
+    e = M.Engine.from_system(W.argon_fcc(30, seed=1, jitter=0.02))
+    e.nonbond()
+    assert e.form() == ("queue", 0, False)
+    warps, layout, stages, occupancy, _ = e.autotune(5)
+
+    def form():
+        e.nonbond()
+        return e.form().name
+
+    assert form() == "cells" and e.form().rows in (24, 32)
+    e.set_layout(layout, stages, occupancy)
+    assert form() == "cells"
+    e.set_layout(1 - layout, 1, 640)
+    assert form() == "queue"
+    e.set_layout(layout, stages, occupancy)
+    assert form() == "cells"
+    e.set_order(e.get_order())
+    assert form() == "queue"
+    e.close()
+
+
+def test_task_clocks_run_the_queue_form(monkeypatch):
+    monkeypatch.setenv("MDB_SWEEP_FORM", "cells")
+    e = M.Engine.from_system(W.argon_fcc(7))
+    e.task_clocks(True)
+    e.nonbond()
+    assert e.form().name == "queue" and (e.task_clocks(True, read=True)[0] > 0).any()
+    e.close()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_on_a_stream_of_the_caller(graph, monkeypatch):
+    """The candidate count's own stream forks from and joins whatever stream is set."""
+    torch = pytest.importorskip("torch")
+    monkeypatch.setenv("MDB_SWEEP_FORM", "cells")
+    sysm = W.argon_fcc(10, seed=2, jitter=0.05)
+    sysm.v = W.maxwell_velocities(sysm, 150.0, seed=3)
+    out = []
+    for stream in (None, torch.cuda.Stream()):
+        e = M.Engine.from_system(sysm)
+        e.graph(graph)
+        if stream:
+            e.set_stream(stream.cuda_stream)
+        for _ in range(4):
+            e.nonbond()
+        counts = e.stats().candidates
+        for _ in range(5):
+            e.step()
+        assert e.form() == ("cells", 32, graph)
+        out.append([counts, e.stats().candidates, *e.parts()])
+        e.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+def test_grouped_batch_steps(monkeypatch):
+    monkeypatch.setenv("MDB_SWEEP_FORM", "cells")
+    out = []
+    for groups in (1, 3):
+        systems = W.argon_replicas(7, seed=5)
+        for k, s in enumerate(systems):
+            s.v = W.maxwell_velocities(s, 100.0, seed=k)
+        engines = [M.Engine.from_system(s, start=False) for s in systems]
+        b = M.Batch(engines)
+        b.set_groups(groups)
+        for _ in range(4):
+            b.step()
+        assert b.form().name == "cells"
+        out.append([b.stats().pairs, b.stats().candidates] + [a for e in engines for a in e.parts()])
+        b.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+def test_shares_of_a_large_cell_in_resident_steps(monkeypatch):
+    """A cell of 1,000 particles: its strips' j particles are split between units, in resident
+    steps as in host-buffer evaluations."""
+    monkeypatch.setenv("MDB_SWEEP_FORM", "cells")
+    sysm = one_large_cell()
+    sysm.v = W.maxwell_velocities(sysm, 50.0, seed=1)
+    out = []
+    for host in (False, True):
+        e = M.Engine.from_system(sysm)
+        if host:
+            for _ in range(5):
+                e.step_host()
+        else:
+            e.resident_begin().resident_steps(5).resident_end()
+        assert e.form().name == "cells"
+        out.append(e.parts())
+        e.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
