@@ -727,6 +727,9 @@ int engine_cuda_setspin(struct engine *e, int polls);
  * the particles were uploaded; -1 without the flag or resident particles. */
 int engine_cuda_verlet_rebuilds(struct engine *e, int *rebuilds);
 int engine_cuda_copytimeout_test(struct engine *e, int enable);
+/* Test hook: room for at most `units` units of the cell form (0: no limit), so that its unit
+ * list overflows: the evaluation then ends with engine_err_maxparts. */
+int engine_cuda_unitcap_test(struct engine *e, int units);
 
 /* ---- batches of engines (no counterpart in the reference) ----
  * One device state for many independent engines (replicas: the same potentials, cutoff

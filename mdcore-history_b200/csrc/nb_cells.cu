@@ -473,7 +473,7 @@ __global__ void __launch_bounds__(kCellWarps * 32 + 32, 1) sweep_cells(CellParam
     __syncthreads();
 
     const bool need_pid = EX || (TAB == kTabGlobal && P.ep_pot >= 0);
-    const int nu = *C.nunits;
+    const int nu = min(*C.nunits, C.units_cap);
     const int batch = max(1, min(4, nu / (8 * (int)gridDim.x * nw)));
     const f32x2 nz2 = pack2(C.neg_zero, C.neg_zero);
     CellSums R;
@@ -791,13 +791,13 @@ cudaError_t launch_cell_count(const CellParams& C, int grid, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_cell_sweep(const CellParams& C, int ncells, int rows, int2* units, size_t units_cap, bool has_excl,
-                              int tab, int nw, size_t smem, int grid, bool capturing, cudaStream_t s) {
+cudaError_t launch_cell_sweep(const CellParams& C, int ncells, int rows, int2* units, bool has_excl, int tab, int nw,
+                              size_t smem, int grid, bool capturing, cudaStream_t s) {
     cudaError_t err = cudaMemsetAsync(C.head, 0, 2 * sizeof(int), s);
     if (err != cudaSuccess) return err;
     const Params& P = C.p;
     cell_units<<<(ncells + 255) / 256, 256, 0, s>>>(P.ccount, C.toff, C.tasks, ncells, rows, units, C.head + 1,
-                                                    (int)units_cap, P.acc, P.abort);
+                                                    C.units_cap, P.acc, P.abort);
     err = cudaGetLastError();
     if (err != cudaSuccess) return err;
     return rows == 24 ? launch_rows<24>(C, has_excl, tab, nw, smem, grid, capturing, s)

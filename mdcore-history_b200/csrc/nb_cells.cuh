@@ -11,7 +11,8 @@ constexpr int kCellSlotBits = 27;        // bits of a slot number in a list entr
 struct CellParams {
     Params p;
     const int2* units;          // cell, strip | strips << 8 | share << 16 | shares << 24
-    const int* nunits;
+    const int* nunits;          // may exceed units_cap (a status bit is set then)
+    int units_cap;              // room in units
     int* head;                  // queue head
     const int* toff;            // tasks of cell c (as its ci): [toff[c], toff[c + 1])
     const TaskRec* tasks;
@@ -30,12 +31,13 @@ size_t cell_units_bound(size_t nslots, int ncells, int cap, int maxtasks);
 // (0: read from global memory), npots tables and mt types; false when they do not fit.
 bool cell_sweep_shape(int rows, int ncoef, int npots, int mt, int* nw, int* copies, size_t* smem);
 
-// rows: i particles of a unit at most, 24 or 32.  Clears the queue words (queue head, number of units), lists the units of the cells' current
-// counts and sweeps them: nw warps per block, one block per SM.  tab: table mode (kTabShared,
-// kTabOne, kTabGlobal).  units has room for units_cap.  The kernels' attributes are set unless
-// the stream is being captured.
-cudaError_t launch_cell_sweep(const CellParams& C, int ncells, int rows, int2* units, size_t units_cap, bool has_excl,
-                              int tab, int nw, size_t smem, int grid, bool capturing, cudaStream_t s);
+// Clears the queue words (queue head, number of units), lists the units of the cells' current
+// counts and sweeps them: nw warps per block, one block per SM.  rows: i particles of a unit at
+// most, 24 or 32.  tab: table mode (kTabShared, kTabOne, kTabGlobal).  units: C.units, with room
+// for C.units_cap; units past it are dropped with kStatusCellOverflow.  The kernels' attributes
+// are set unless the stream is being captured.
+cudaError_t launch_cell_sweep(const CellParams& C, int ncells, int rows, int2* units, bool has_excl, int tab, int nw,
+                              size_t smem, int grid, bool capturing, cudaStream_t s);
 
 // Counts the sorted sweep's candidates when *C.count_cand (one block per SM).
 cudaError_t launch_cell_count(const CellParams& C, int grid, cudaStream_t s);

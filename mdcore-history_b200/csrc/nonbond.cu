@@ -95,6 +95,7 @@ struct NbState {
     float4* d_cshift = nullptr;
     int2* d_units = nullptr;       // units of the evaluation, their number and the queue head
     size_t units_cap = 0;
+    size_t units_cap_test = INT_MAX;   // test hook (engine_cuda_unitcap_test)
     int* d_unit_words = nullptr;   // queue head, units, count candidates (resident steps), 1
     // The sort keys of a buffer (d_keys, r_keys) are not its last evaluation's: none has been
     // sorted there yet, or the last one ran in the cell form.
@@ -726,6 +727,7 @@ int launch_cells(NbState* st, const Params& P, const int* count_cand) {
     C.p = P;
     C.units = st->d_units;
     C.nunits = st->d_unit_words + 1;
+    C.units_cap = (int)std::min(st->units_cap, st->units_cap_test);
     C.head = st->d_unit_words;
     C.toff = st->d_toff;
     C.tasks = st->d_ctasks;
@@ -738,7 +740,7 @@ int launch_cells(NbState* st, const Params& P, const int* count_cand) {
     cell_shape(st, &nw, &C.copies, &smem);
     CU(cudaEventRecord(st->ev_fork, st->stream));
     CU(cudaStreamWaitEvent(st->side_stream, st->ev_fork, 0));
-    CU(launch_cell_sweep(C, st->ncells, st->cell_rows, st->d_units, st->units_cap, st->has_excl,
+    CU(launch_cell_sweep(C, st->ncells, st->cell_rows, st->d_units, st->has_excl,
                          st->tab_global ? kTabGlobal : st->one_pot ? kTabOne : kTabShared, nw, smem, st->sm_count,
                          st->capturing, st->stream));
     CU(launch_cell_count(C, st->sm_count, st->side_stream));
@@ -2839,6 +2841,17 @@ extern "C" int engine_cuda_setspin(struct engine* e, int polls) {
 // arrive on their staging mbarriers nor issue a copy, so every wait runs out after the spin
 // limit, the evaluation fails with engine_err_cuda ("Bulk copy into shared memory timed
 // out.") and nothing is in flight; 0 restores normal copies.
+// Test hook: room for `units` units of the cell form (0: as many as there can be), so that the
+// list overflows.
+extern "C" int engine_cuda_unitcap_test(struct engine* e, int units) {
+    if (e == nullptr || e->cuda == nullptr) return engine_err_null;
+    if (units < 0) return engine_err_range;
+    NbState* st = state(e);
+    st->units_cap_test = units > 0 ? (size_t)units : (size_t)INT_MAX;
+    ++st->buf_gen;                     // graphs hold the old limit
+    return 0;
+}
+
 extern "C" int engine_cuda_copytimeout_test(struct engine* e, int enable) {
     if (e == nullptr || e->cuda == nullptr) return engine_err_null;
     if (enable != 0 && enable != 1) return engine_err_range;

@@ -174,6 +174,7 @@ def lib() -> C.CDLL:
         "engine_cuda_setspin": (C.c_int, [vp, C.c_int]),
         "engine_cuda_verlet_rebuilds": (C.c_int, [vp, ip]),
         "engine_cuda_copytimeout_test": (C.c_int, [vp, C.c_int]),
+        "engine_cuda_unitcap_test": (C.c_int, [vp, C.c_int]),
         "engine_sched_record": (C.c_int, [vp, C.c_int]),
         "engine_sched_features": (C.c_int, [vp, P(C.c_float), C.c_int]),
         "engine_sched_targets": (C.c_int, [vp, P(C.c_float), C.c_int]),
@@ -432,6 +433,11 @@ class Engine:
     def copytimeout_test(self, enable: bool):
         """Test hook: the sweeps' staging copies are not issued, so their waits run out."""
         _check(self.lib.engine_cuda_copytimeout_test(self.ptr, int(enable)), "engine_cuda_copytimeout_test")
+        return self
+
+    def unitcap_test(self, units: int):
+        """Test hook: room for at most `units` units of the cell form (0: no limit)."""
+        _check(self.lib.engine_cuda_unitcap_test(self.ptr, units), "engine_cuda_unitcap_test")
         return self
 
     def load_parts(self):

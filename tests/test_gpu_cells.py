@@ -326,3 +326,29 @@ def test_shares_of_a_large_cell_in_resident_steps(monkeypatch):
         out.append(e.parts())
         e.close()
     assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_an_overflowing_unit_list_is_an_error(graph, monkeypatch):
+    """Units past the list's room are dropped and reported, and none past it is read."""
+    monkeypatch.setenv("MDB_SWEEP_FORM", "cells")
+    sysm = W.argon_fcc(10, seed=2, jitter=0.05)
+    e = M.Engine.from_system(sysm)
+    e.graph(graph)
+    for _ in range(3):
+        e.nonbond()
+    f, pairs = e.forces(), e.stats().pairs
+    for units in (1, 50):
+        e.unitcap_test(units)
+        for _ in range(3):
+            with pytest.raises(M.MdcoreError, match="Max. number of parts per cell"):
+                e.nonbond()
+            assert e.stats().status == 2 and 0 < e.stats().pairs < pairs
+    e.unitcap_test(0)
+    for _ in range(3):
+        e.nonbond()
+        assert np.array_equal(e.forces(), f) and e.stats().pairs == pairs
+    e.unitcap_test(1)
+    with pytest.raises(M.MdcoreError, match="Max. number of parts per cell"):
+        e.step()
+    e.close()
