@@ -727,9 +727,10 @@ int engine_cuda_setspin(struct engine *e, int polls);
  * the particles were uploaded; -1 without the flag or resident particles. */
 int engine_cuda_verlet_rebuilds(struct engine *e, int *rebuilds);
 int engine_cuda_copytimeout_test(struct engine *e, int enable);
-/* Test hook: room for at most `units` units of the cell form (0: no limit), so that its unit
- * list overflows: the evaluation then ends with engine_err_maxparts. */
-int engine_cuda_unitcap_test(struct engine *e, int units);
+/* Test hook: lower limits of the cell form (0: its own).  units: room in its unit list, past which
+ * an evaluation ends with engine_err_maxparts; slots: particle slots (2^27) of an evaluation, past
+ * which it runs in the queue form. */
+int engine_cuda_celllimits_test(struct engine *e, int units, int slots);
 
 /* ---- batches of engines (no counterpart in the reference) ----
  * One device state for many independent engines (replicas: the same potentials, cutoff

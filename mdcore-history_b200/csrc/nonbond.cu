@@ -95,7 +95,8 @@ struct NbState {
     float4* d_cshift = nullptr;
     int2* d_units = nullptr;       // units of the evaluation, their number and the queue head
     size_t units_cap = 0;
-    size_t units_cap_test = INT_MAX;   // test hook (engine_cuda_unitcap_test)
+    // Limits of the cell form; lower ones by a test hook (engine_cuda_celllimits_test).
+    size_t units_most = INT_MAX, cell_slots = (size_t)1 << kCellSlotBits;
     int* d_unit_words = nullptr;   // queue head, units, count candidates (resident steps), 1
     // The sort keys of a buffer (d_keys, r_keys) are not its last evaluation's: none has been
     // sorted there yet, or the last one ran in the cell form.
@@ -704,7 +705,9 @@ std::atomic<int> copy_hook[kHookDevices];
 // hundred steps of such systems (close contacts of a random vapour, truncated charges, the
 // constraint iterations) that last bit grows to per mille of the velocities, as it does
 // between the queue form's own lane layouts; a single table's trajectories keep five digits.
-bool use_cells(const NbState* st, bool steps) {
+// slots: particle slots of the evaluation (list entries hold kCellSlotBits of a slot's number).
+bool use_cells(const NbState* st, bool steps, size_t slots) {
+    if (slots > st->cell_slots) return false;
     if (!st->cells_ok || st->queue_form || st->plain || st->record_clock || st->unsorted) return false;
     if (steps && !st->one_pot && !st->cells_forced) return false;
     if (st->device >= 0 && st->device < kHookDevices && copy_hook[st->device].load() != 0) return false;
@@ -712,6 +715,10 @@ bool use_cells(const NbState* st, bool steps) {
         if (!(e->flags & engine_flag_verlet)) return true;
     return false;
 }
+
+// Particle slots of a host-buffer evaluation and of a resident step.
+size_t host_slots(const NbState* st) { return (size_t)st->h_cstart[st->ncells]; }
+size_t res_slots(const NbState* st) { return (size_t)st->ncells * st->capc; }
 
 // Worker warps, table copies and shared memory of the cell form for the state's tables.
 bool cell_shape(const NbState* st, int* nw, int* copies, size_t* smem) {
@@ -727,7 +734,7 @@ int launch_cells(NbState* st, const Params& P, const int* count_cand) {
     C.p = P;
     C.units = st->d_units;
     C.nunits = st->d_unit_words + 1;
-    C.units_cap = (int)std::min(st->units_cap, st->units_cap_test);
+    C.units_cap = (int)std::min(st->units_cap, st->units_most);
     C.head = st->d_unit_words;
     C.toff = st->d_toff;
     C.tasks = st->d_ctasks;
@@ -838,7 +845,7 @@ DevView host_view(const NbState* st) {
 // Bookkeeping of an evaluation being issued directly or as a graph: its form, and whether the
 // sort keys of its buffer are its own (the cell form sorts nothing).  steps: of a time step.
 void note_evaluation(NbState* st, bool resident, bool steps, bool graph) {
-    const bool cells = use_cells(st, steps);
+    const bool cells = use_cells(st, steps, resident ? res_slots(st) : host_slots(st));
     (resident ? st->res_keys_stale : st->host_keys_stale) = cells;
     st->last_form = cells ? engine_cuda_form_cells : st->plain ? engine_cuda_form_plain : engine_cuda_form_queue;
     st->last_rows = cells ? st->cell_rows : 0;
@@ -864,7 +871,7 @@ int issue_kernels(NbState* st, const DevView& V, bool span = true) {
         if (rc == 0 && span) rc = record_event(st, st->ev1);
         return rc;
     }
-    const bool cells = use_cells(st, V.resident || st->stepping);
+    const bool cells = use_cells(st, V.resident || st->stepping, V.slots);
     if (!cells) {
         const int rc0 = launch_sort(V.xq, V.cstart, V.ccount, st->d_cmask, V.keys, st->d_cscale, st->ncells, V.cpc, cap,
                                     st->d_acc, V.abort, st->capturing, st->stream, V.rebuild);
@@ -981,7 +988,7 @@ long long launch_key(const NbState* st) {
     k = k * 3 + st->plain;
     k = k * 3 + st->record_clock;
     k = k * 2 + st->fp32acc;
-    k = k * 4 + (use_cells(st, st->stepping) ? st->cell_rows / 8 - 2 : 0);
+    k = k * 4 + (use_cells(st, st->stepping, host_slots(st)) ? st->cell_rows / 8 - 2 : 0);
     return k;
 }
 
@@ -1395,13 +1402,13 @@ int load_state(NbState* st) {
     CU(cudaMemcpy(st->d_exlist, exlist.data(), exlist.size() * sizeof(int), cudaMemcpyHostToDevice));
     // Engines that evaluate in the cell form from the start have its lists before their first
     // evaluation, like everything above.
-    if (use_cells(st, false)) {
-        size_t slots = 4;
-        int most = 0;
-        for (const struct cell* c : st->flat_cells) {
-            slots += (size_t)((c->count + 3) & ~3);
-            most = std::max(most, c->count);
-        }
+    size_t slots = 4;
+    int most = 0;
+    for (const struct cell* c : st->flat_cells) {
+        slots += (size_t)((c->count + 3) & ~3);
+        most = std::max(most, c->count);
+    }
+    if (use_cells(st, false, slots)) {
         int rc = build_cell_tasks(st);
         if (rc == 0) rc = reserve_units(st, slots, (std::min(most, kMaxPartsPerCell) + 3) & ~3);
         if (rc < 0) return rc;
@@ -1669,7 +1676,7 @@ int st_autotune(NbState* st, int reps, int* warps_out, int* layout_out, int* sta
     // resident steps take once per call only.
     st->queue_form = false;
     int best_rows = 0;
-    if (use_cells(st, false) && (st->one_pot || st->tab_global || st->cells_forced)) {
+    if (use_cells(st, false, host_slots(st)) && (st->one_pot || st->tab_global || st->cells_forced)) {
         cudaError_t err = cudaMemsetAsync(st->d_unit_words + 3, 0, sizeof(int), st->stream);
         int rc = 0;
         for (int rows = 32; rows >= 24 && rc == 0 && err == cudaSuccess; rows -= 8) {
@@ -1998,7 +2005,6 @@ int res_alloc(NbState* st, int capc, int mcap, long long n) {
     st->mcap = mcap;
     st->res_nparts = n;
     const size_t slots = (size_t)nc * st->capc;
-    if (slots >> kCellSlotBits) st->cells_ok = false;      // beyond the cell form's slot numbers
     for (int q = 0; q < 2; q++) {
         CU(cudaMalloc(&st->r_xq[q], sizeof(float4) * slots));
         CU(cudaMalloc(&st->r_v[q], sizeof(float4) * slots));
@@ -2372,7 +2378,7 @@ long long res_key(const NbState* st) {
     k = k * 2 + (st->sd_gamma > 0.f);
     k = k * 2 + (st->elog_cap > 0);
     k = k * 2 + st->verlet;
-    k = k * 4 + (use_cells(st, true) ? st->cell_rows / 8 - 2 : 0);
+    k = k * 4 + (use_cells(st, true, res_slots(st)) ? st->cell_rows / 8 - 2 : 0);
     return k;
 }
 
@@ -2841,14 +2847,16 @@ extern "C" int engine_cuda_setspin(struct engine* e, int polls) {
 // arrive on their staging mbarriers nor issue a copy, so every wait runs out after the spin
 // limit, the evaluation fails with engine_err_cuda ("Bulk copy into shared memory timed
 // out.") and nothing is in flight; 0 restores normal copies.
-// Test hook: room for `units` units of the cell form (0: as many as there can be), so that the
-// list overflows.
-extern "C" int engine_cuda_unitcap_test(struct engine* e, int units) {
+// Test hook: lower limits of the cell form (0: its own), units of an evaluation and particle
+// slots of one that runs in it.
+extern "C" int engine_cuda_celllimits_test(struct engine* e, int units, int slots) {
     if (e == nullptr || e->cuda == nullptr) return engine_err_null;
-    if (units < 0) return engine_err_range;
+    if (units < 0 || slots < 0) return engine_err_range;
     NbState* st = state(e);
-    st->units_cap_test = units > 0 ? (size_t)units : (size_t)INT_MAX;
-    ++st->buf_gen;                     // graphs hold the old limit
+    st->units_most = units > 0 ? (size_t)units : (size_t)INT_MAX;
+    st->cell_slots = (size_t)1 << kCellSlotBits;
+    if (slots > 0) st->cell_slots = std::min(st->cell_slots, (size_t)slots);
+    ++st->buf_gen;                     // graphs hold the old limit of units
     return 0;
 }
 

@@ -174,7 +174,7 @@ def lib() -> C.CDLL:
         "engine_cuda_setspin": (C.c_int, [vp, C.c_int]),
         "engine_cuda_verlet_rebuilds": (C.c_int, [vp, ip]),
         "engine_cuda_copytimeout_test": (C.c_int, [vp, C.c_int]),
-        "engine_cuda_unitcap_test": (C.c_int, [vp, C.c_int]),
+        "engine_cuda_celllimits_test": (C.c_int, [vp, C.c_int, C.c_int]),
         "engine_sched_record": (C.c_int, [vp, C.c_int]),
         "engine_sched_features": (C.c_int, [vp, P(C.c_float), C.c_int]),
         "engine_sched_targets": (C.c_int, [vp, P(C.c_float), C.c_int]),
@@ -435,9 +435,9 @@ class Engine:
         _check(self.lib.engine_cuda_copytimeout_test(self.ptr, int(enable)), "engine_cuda_copytimeout_test")
         return self
 
-    def unitcap_test(self, units: int):
-        """Test hook: room for at most `units` units of the cell form (0: no limit)."""
-        _check(self.lib.engine_cuda_unitcap_test(self.ptr, units), "engine_cuda_unitcap_test")
+    def celllimits_test(self, units: int = 0, slots: int = 0):
+        """Test hook: lower limits of the cell form, units and particle slots (0: its own)."""
+        _check(self.lib.engine_cuda_celllimits_test(self.ptr, units, slots), "engine_cuda_celllimits_test")
         return self
 
     def load_parts(self):

@@ -339,16 +339,48 @@ def test_an_overflowing_unit_list_is_an_error(graph, monkeypatch):
         e.nonbond()
     f, pairs = e.forces(), e.stats().pairs
     for units in (1, 50):
-        e.unitcap_test(units)
+        e.celllimits_test(units=units)
         for _ in range(3):
             with pytest.raises(M.MdcoreError, match="Max. number of parts per cell"):
                 e.nonbond()
             assert e.stats().status == 2 and 0 < e.stats().pairs < pairs
-    e.unitcap_test(0)
+    e.celllimits_test()
     for _ in range(3):
         e.nonbond()
         assert np.array_equal(e.forces(), f) and e.stats().pairs == pairs
-    e.unitcap_test(1)
+    e.celllimits_test(units=1)
     with pytest.raises(M.MdcoreError, match="Max. number of parts per cell"):
         e.step()
+    e.close()
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_more_slots_than_the_cell_form_numbers(graph, monkeypatch):
+    """The slot limit (lowered here) is looked at for every evaluation on its own, on host buffers
+    and in resident blocks, and blocks past it do not switch the form off for later ones."""
+    monkeypatch.setenv("MDB_SWEEP_FORM", "cells")
+    e = M.Engine.from_system(W.argon_fcc(10, seed=2, jitter=0.05))
+    e.graph(graph)
+    slots = int(((np.bincount(e.cells()) + 3) // 4 * 4).sum())
+
+    def forms():
+        out = []
+        for _ in range(3):
+            e.nonbond()
+            out.append(e.form().name)
+        for margin in (0, 400):
+            e.resident_begin(margin)
+            e.resident_steps(5)
+            out.append(e.form().name)
+            e.resident_end()
+        return out
+
+    assert forms() == ["cells"] * 5
+    e.celllimits_test(slots=slots // 2)
+    assert forms() == ["queue"] * 5
+    e.celllimits_test(slots=3 * slots)
+    assert forms() == ["cells"] * 4 + ["queue"]
+    assert forms() == ["cells"] * 4 + ["queue"]
+    e.celllimits_test()
+    assert forms() == ["cells"] * 5
     e.close()
