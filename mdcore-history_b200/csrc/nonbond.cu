@@ -82,7 +82,8 @@ struct NbState {
     // task lists fit it and nothing asks for the task queue (queue_form), see use_cells.
     bool cells_ok = false;
     bool queue_form = false;
-    bool cells_forced = false;     // MDB_SWEEP_FORM=cells: time steps of every system too
+    // MDB_SWEEP_FORM: the autotuner leaves the form alone; cells serve time steps of every system too
+    bool queue_forced = false, cells_forced = false;
     bool stepping = false;         // a host-buffer evaluation is part of a time step
     int cell_rows = 32;            // i particles of a unit of the cell form (24 or 32)
     bool tuned = false;            // autotuned: tuned_shape, tuned_cells are its choice
@@ -1315,7 +1316,8 @@ int load_state(NbState* st) {
         // form alone and in a batch.  MDB_SWEEP_FORM=queue, cells or cells24 overrides.
         const char* form = std::getenv("MDB_SWEEP_FORM");
         st->cells_forced = form && std::strncmp(form, "cells", 5) == 0;
-        st->queue_form = form ? std::strncmp(form, "cells", 5) != 0 : !st->tab_global;
+        st->queue_forced = form && !st->cells_forced;
+        st->queue_form = form ? st->queue_forced : !st->tab_global;
         st->cell_rows = form ? (std::strcmp(form, "cells24") == 0 ? 24 : 32) : st->tab_global ? 24 : 32;
     }
     if (dev_alloc(&st->d_tasks, tasks.size()) || dev_alloc(&st->d_tshift, tshift.size())) return engine_err_cuda;
@@ -1676,10 +1678,13 @@ int st_autotune(NbState* st, int reps, int* warps_out, int* layout_out, int* sta
     // resident steps take once per call only.
     st->queue_form = false;
     int best_rows = 0;
-    if (use_cells(st, false, host_slots(st)) && (st->one_pot || st->tab_global || st->cells_forced)) {
+    if (!st->queue_forced && use_cells(st, false, host_slots(st)) &&
+        (st->one_pot || st->tab_global || st->cells_forced)) {
+        const int only = st->cells_forced ? st->cell_rows : 0;     // MDB_SWEEP_FORM's rows
         cudaError_t err = cudaMemsetAsync(st->d_unit_words + 3, 0, sizeof(int), st->stream);
         int rc = 0;
         for (int rows = 32; rows >= 24 && rc == 0 && err == cudaSuccess; rows -= 8) {
+            if (only && rows != only) continue;
             st->cell_rows = rows;
             std::vector<float> t;
             for (int r = 0; r <= reps && rc == 0 && err == cudaSuccess; r++) {
@@ -1692,7 +1697,7 @@ int st_autotune(NbState* st, int reps, int* warps_out, int* layout_out, int* sta
             }
             if (rc < 0 || err != cudaSuccess) break;
             std::sort(t.begin(), t.end());
-            if (t[t.size() / 2] < best_ms) {
+            if (only || t[t.size() / 2] < best_ms) {
                 best_ms = t[t.size() / 2];
                 best_rows = rows;
             }

@@ -384,3 +384,23 @@ def test_more_slots_than_the_cell_form_numbers(graph, monkeypatch):
     e.celllimits_test()
     assert forms() == ["cells"] * 5
     e.close()
+
+
+@pytest.mark.parametrize("form", ["queue", "cells", "cells24"])
+@pytest.mark.parametrize("ncell", [7, 30])
+def test_the_autotuner_keeps_the_form_asked_for(form, ncell, monkeypatch):
+    """MDB_SWEEP_FORM overrides the autotuner's choice (by itself the queue form for the small
+    system, the cell form for the large one)."""
+    monkeypatch.setenv("MDB_SWEEP_FORM", form)
+    e = M.Engine.from_system(W.argon_fcc(ncell, seed=1, jitter=0.02))
+    _, layout, stages, occupancy, _ = e.autotune(3)
+    want = {"queue": ("queue", 0), "cells": ("cells", 32), "cells24": ("cells", 24)}[form]
+    assert e.form()[:2] == want
+    e.nonbond()
+    assert e.form()[:2] == want
+    e.step()
+    assert e.form()[:2] == want
+    e.set_layout(layout, stages, occupancy)
+    e.nonbond()
+    assert e.form()[:2] == want
+    e.close()
