@@ -1627,10 +1627,43 @@ int st_autotune(NbState* st, int reps, int* warps_out, int* layout_out, int* sta
     }
     CU(cudaSetDevice(st->device));
     if (reps < 1) reps = 1;
-    const bool graph = st->use_graph;
+    // Restored when an evaluation fails; kept settings overwrite it.
+    struct Settings {
+        bool graph, queue_form;
+        int plain, warps, layout, stages, occupancy, window, rows;
+    } const was = {st->use_graph, st->queue_form, st->plain,  st->warps,    st->layout,
+                   st->stages,    st->occupancy,  st->window, st->cell_rows};
+    auto restore = [&](int rc) {
+        st->use_graph = was.graph;
+        st->queue_form = was.queue_form;
+        st->plain = was.plain;
+        st->warps = was.warps;
+        st->layout = was.layout;
+        st->stages = was.stages;
+        st->occupancy = was.occupancy;
+        st->window = was.window;
+        st->cell_rows = was.rows;
+        return rc;
+    };
+    // Median device time of reps evaluations after one warm-up; negative: an error code.
+    auto median_ms = [&](float* ms) -> int {
+        std::vector<float> t;
+        for (int r = 0; r <= reps; r++) {
+            const int rc = st_resident(st);
+            if (rc < 0) return rc;
+            CU(cudaEventSynchronize(st->ev1));
+            float one = 0.f;
+            CU(cudaEventElapsedTime(&one, st->ev0, st->ev1));
+            if (r > 0) t.push_back(one);
+        }
+        std::sort(t.begin(), t.end());
+        *ms = t[t.size() / 2];
+        return 0;
+    };
     st->use_graph = false;
     st->plain = 0;
     st->queue_form = true;
+    st->window = 4;
     // warps, layout, stages, threads per SM (window 4: the 8-step window was never the
     // fastest shape)
     static const int shapes[][4] = {
@@ -1647,74 +1680,47 @@ int st_autotune(NbState* st, int reps, int* warps_out, int* layout_out, int* sta
         st->layout = shapes[k][1];
         st->stages = shapes[k][2];
         st->occupancy = shapes[k][3];
-        st->window = 4;
-        std::vector<float> t;
-        for (int r = 0; r <= reps; r++) {
-            int rc = st_resident(st);
-            if (rc < 0) {
-                st->use_graph = graph;
-                return rc;
-            }
-            CU(cudaEventSynchronize(st->ev1));
-            float ms = 0.f;
-            CU(cudaEventElapsedTime(&ms, st->ev0, st->ev1));
-            if (r > 0) t.push_back(ms);
-        }
-        std::sort(t.begin(), t.end());
-        const float med = t[t.size() / 2];
-        if (best < 0 || med < best_ms) {
+        float ms = 0.f;
+        const int rc = median_ms(&ms);
+        if (rc < 0) return restore(rc);
+        if (best < 0 || ms < best_ms) {
             best = k;
-            best_ms = med;
+            best_ms = ms;
         }
     }
     st->warps = shapes[best][0];
     st->layout = shapes[best][1];
     st->stages = shapes[best][2];
     st->occupancy = shapes[best][3];
-    st->window = 4;
     // The cell form with units of 32 and of 24 rows, for the systems whose steps or default
     // evaluations may run it; kept when it beats the queue form's best (whose shape is the one
-    // returned).  It is timed without its candidate count, which
-    // resident steps take once per call only.
+    // returned).  It is timed as force evaluations and steps of one per call run it, with its
+    // candidate count (only the last of several steps in a call counts): timed without, it was
+    // kept for argon of 32,000 atoms (0.061 against 0.066 ms), whose evaluations then took 0.075
+    // ms and single steps 0.116 instead of 0.104.
     st->queue_form = false;
     int best_rows = 0;
     if (!st->queue_forced && use_cells(st, false, host_slots(st)) &&
         (st->one_pot || st->tab_global || st->cells_forced)) {
         const int only = st->cells_forced ? st->cell_rows : 0;     // MDB_SWEEP_FORM's rows
-        cudaError_t err = cudaMemsetAsync(st->d_unit_words + 3, 0, sizeof(int), st->stream);
-        int rc = 0;
-        for (int rows = 32; rows >= 24 && rc == 0 && err == cudaSuccess; rows -= 8) {
+        for (int rows = 32; rows >= 24; rows -= 8) {
             if (only && rows != only) continue;
             st->cell_rows = rows;
-            std::vector<float> t;
-            for (int r = 0; r <= reps && rc == 0 && err == cudaSuccess; r++) {
-                rc = st_resident(st);
-                if (rc < 0) break;
-                err = cudaEventSynchronize(st->ev1);
-                float ms = 0.f;
-                if (err == cudaSuccess) err = cudaEventElapsedTime(&ms, st->ev0, st->ev1);
-                if (r > 0) t.push_back(ms);
-            }
-            if (rc < 0 || err != cudaSuccess) break;
-            std::sort(t.begin(), t.end());
-            if (only || t[t.size() / 2] < best_ms) {
-                best_ms = t[t.size() / 2];
+            float ms = 0.f;
+            const int rc = median_ms(&ms);
+            if (rc < 0) return restore(rc);
+            if (only || ms < best_ms) {
+                best_ms = ms;
                 best_rows = rows;
             }
         }
-        if (err == cudaSuccess) err = cudaMemsetAsync(st->d_unit_words + 3, 1, sizeof(int), st->stream);
-        if (rc < 0 || err != cudaSuccess) {
-            st->use_graph = graph;
-            CU(err);
-            return rc;
-        }
     }
     st->queue_form = best_rows == 0;
-    if (best_rows) st->cell_rows = best_rows;
+    st->cell_rows = best_rows ? best_rows : was.rows;
     st->tuned = true;
     st->tuned_cells = !st->queue_form;
     for (int k = 0; k < 4; k++) st->tuned_shape[k] = shapes[best][k];
-    st->use_graph = graph;
+    st->use_graph = was.graph;
     const int rc = st_resident(st);           // leave the chosen form's results resident
     if (rc < 0) return rc;
     if (warps_out) *warps_out = st->warps;
