@@ -585,8 +585,9 @@ int engine_sched_apply(struct engine *e, int use_mlp);
 int engine_sched_order(struct engine *e, int source, int tile);
 /* The current queue order (n = the task count). */
 int engine_cuda_getorder(struct engine *e, int *order, int n);
-/* Sweep kernel launch parameters: warps per block (0 = default) and plain = 1 for the
- * plain form (one block per task, IEEE sqrt/div) instead of the persistent queue. */
+/* Sweep kernel launch parameters: warps per block (0 = default; any other count selects the
+ * queue form, see engine_cuda_autotune) and plain = 1 for the plain form (one block per task,
+ * IEEE sqrt/div) instead of the persistent forms. */
 int engine_cuda_settune(struct engine *e, int warps, int plain);
 /* Replaces the device task-queue order (a permutation of 0..ntasks-1). */
 int engine_cuda_setorder(struct engine *e, const int *order, int n);
@@ -641,15 +642,18 @@ int engine_cuda_setlayout(struct engine *e, int layout, int stages, int occupanc
  * (uploaded first if none are) and keeps the fastest; for systems with one table for every
  * pair of types, or with tables that do not fit in shared memory, also the cell form (units of
  * up to 24 or 32 particles of a cell against all its neighbours at once, no sort).  Returns
- * the best queue shape and the median device time of what was kept.  Results stay resident.
+ * the best queue shape and the median device time of an evaluation in the form that was kept
+ * (engine_cuda_getform).  Results stay resident.
  * Both forms give the same pair, exclusion and candidate counts and forces within FP32
  * rounding of their sums.  Time steps run the cell form only with one table (elsewhere
- * trajectories amplify the other order of sums).  Passing the returned shape to
- * engine_cuda_setlayout keeps the choice; any other shape, or a queue order given afterwards
- * (engine_cuda_setorder, engine_sched_order, engine_sched_apply), selects the queue form.
+ * trajectories amplify the other order of sums).  Launch shapes and queue orders are about the
+ * queue form: a warp count other than 0 (engine_cuda_settune), a window (engine_cuda_setwindow),
+ * a layout (engine_cuda_setlayout), or an order given after the autotuner (engine_cuda_setorder,
+ * engine_sched_order, engine_sched_apply) selects it.  A shape that is the one returned here
+ * (window 4) stands for the autotuner's choice, and giving it brings that choice back.
  * Without the autotuner: the queue form, and for force evaluations of systems whose tables do
- * not fit in shared memory the cell form; the environment variable MDB_SWEEP_FORM (queue,
- * cells, cells24), read when the device state is built, overrides, for time steps too. */
+ * not fit in shared memory the cell form.  The environment variable MDB_SWEEP_FORM (queue,
+ * cells, cells24), read when the device state is built, overrides both, for time steps too. */
 int engine_cuda_autotune(struct engine *e, int reps, int *warps, int *layout, int *stages, int *occupancy,
                          float *ms);
 

@@ -66,6 +66,7 @@ struct NbState {
     int npots = 0, ncoef = 0, max_type = 0;
     // tuning
     int warps = 4;
+    int warps_asked = 0;           // the count last given (engine_cuda_settune), 0: none
     int window = 4;                // sweep steps per register reduce-scatter (4 or 8)
     int layout = 0;                // persistent sweep: 0 = 32 i per warp, 1 = 8 i x 4 j tile
     int stages = 1;                // staging buffers per worker warp (2: next task's copies in flight)
@@ -699,7 +700,7 @@ constexpr int kHookDevices = 64;
 std::atomic<int> copy_hook[kHookDevices];
 
 // Whether an evaluation runs in the cell form: not when the queue form is asked for (a launch
-// shape, or a queue order given after the autotuner), when per-task clocks are recorded, for
+// shape, see shape_given, or a queue order given after the autotuner), when per-task clocks are recorded, for
 // the unsorted sweep (its candidates are all pairs) or with a Verlet skin (its keys are kept
 // between steps and bound the sweep).  Time steps (steps) of systems of several tables stay in
 // the queue form: the two forms add a particle's pair forces in another order, and over some
@@ -1608,10 +1609,20 @@ int st_kernel_times(NbState* st, float* total_ms, float* sweep_ms) {
     return 0;
 }
 
+// After a launch shape (or a part of one) has been given: a shape is one of the queue form and
+// selects it, the shape the autotuner returned stands for its choice.
+void shape_given(NbState* st) {
+    const int* t = st->tuned_shape;
+    st->queue_form = !(st->tuned_cells && (st->warps_asked == 0 || st->warps_asked == t[0]) && st->layout == t[1] &&
+                       st->stages == t[2] && st->occupancy == t[3] && st->window == 4);
+}
+
 int st_settune(NbState* st, int warps, int plain) {
     if (warps != 0 && warps != 1 && warps != 2 && warps != 4 && warps != 8) return engine_err_range;
     st->warps = warps ? warps : 4;
+    st->warps_asked = warps;
     st->plain = plain ? 1 : 0;
+    if (warps) shape_given(st);
     return 0;
 }
 
@@ -1630,14 +1641,15 @@ int st_autotune(NbState* st, int reps, int* warps_out, int* layout_out, int* sta
     // Restored when an evaluation fails; kept settings overwrite it.
     struct Settings {
         bool graph, queue_form;
-        int plain, warps, layout, stages, occupancy, window, rows;
-    } const was = {st->use_graph, st->queue_form, st->plain,  st->warps,    st->layout,
-                   st->stages,    st->occupancy,  st->window, st->cell_rows};
+        int plain, warps, asked, layout, stages, occupancy, window, rows;
+    } const was = {st->use_graph, st->queue_form, st->plain,     st->warps,  st->warps_asked,
+                   st->layout,    st->stages,     st->occupancy, st->window, st->cell_rows};
     auto restore = [&](int rc) {
         st->use_graph = was.graph;
         st->queue_form = was.queue_form;
         st->plain = was.plain;
         st->warps = was.warps;
+        st->warps_asked = was.asked;
         st->layout = was.layout;
         st->stages = was.stages;
         st->occupancy = was.occupancy;
@@ -1664,6 +1676,7 @@ int st_autotune(NbState* st, int reps, int* warps_out, int* layout_out, int* sta
     st->plain = 0;
     st->queue_form = true;
     st->window = 4;
+    st->warps_asked = 0;
     // warps, layout, stages, threads per SM (window 4: the 8-step window was never the
     // fastest shape)
     static const int shapes[][4] = {
@@ -2792,6 +2805,7 @@ extern "C" int engine_cuda_setwindow(struct engine* e, int window) {
     if (e == nullptr || e->cuda == nullptr) return engine_err_null;
     if (window != 4 && window != 8) return engine_err_range;
     state(e)->window = window;
+    shape_given(state(e));
     return 0;
 }
 
@@ -2802,9 +2816,7 @@ static int st_setlayout(NbState* st, int layout, int stages, int occupancy) {
     st->layout = layout;
     st->stages = stages;
     st->occupancy = occupancy;
-    // A shape is one of the queue form; the shape the autotuner returned stands for its choice.
-    st->queue_form = !(st->tuned_cells && layout == st->tuned_shape[1] && stages == st->tuned_shape[2] &&
-                       occupancy == st->tuned_shape[3]);
+    shape_given(st);
     return 0;
 }
 

@@ -254,7 +254,34 @@ def test_autotuner_choice_and_what_undoes_it():
     assert form() == "cells"
     e.set_order(e.get_order())
     assert form() == "queue"
+    for other, same in (((e.tune, 4 if warps != 4 else 8), (e.tune, warps)), ((e.set_window, 8), (e.set_window, 4))):
+        other[0](other[1])
+        assert form() == "queue"
+        e.set_layout(layout, stages, occupancy)
+        assert form() == "queue"              # not the whole shape
+        same[0](same[1])
+        assert form() == "cells"
+    e.tune(0, plain=True)
+    assert form() == "plain"
+    e.tune(0)
+    assert form() == "cells"
     e.close()
+
+
+def test_launch_shapes_select_the_queue_form_untuned():
+    """An engine whose evaluations run the cell form by default."""
+    for give in (lambda e: e.tune(8), lambda e: e.tune(4), lambda e: e.set_window(8), lambda e: e.set_layout(1),
+                 lambda e: e.set_layout(0)):
+        e = M.Engine.from_system(chain_mix())
+        e.nonbond()
+        assert e.form().name == "cells"
+        e.tune(0)
+        e.nonbond()
+        assert e.form().name == "cells"
+        give(e)
+        e.nonbond()
+        assert e.form().name == "queue"
+        e.close()
 
 
 def test_task_clocks_run_the_queue_form(monkeypatch):
