@@ -136,9 +136,12 @@ struct NbState {
     bool capturing = false;
     int last_grid = 0;             // grid of the last direct persistent launch
     int buf_gen = 0;               // bumped whenever device buffers move
-    long long graph_key = -1, prepared_key = -1;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t graph_exec = nullptr;
+    // One graph per form: force evaluations and host-threaded steps of one engine can differ in it.
+    struct EvalGraph {
+        long long key = -1, prepared = -1;
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+    } eval_graph[2];                // task queue (or plain), cells
     // device buffers
     float4* d_xq = nullptr;
     int* d_pid = nullptr;
@@ -969,12 +972,16 @@ int sort_stale_keys(NbState* st, const DevView& V) {
     return rc;
 }
 
-void drop_graph(NbState* st) {
-    if (st->graph_exec) cudaGraphExecDestroy(st->graph_exec);
-    if (st->graph) cudaGraphDestroy(st->graph);
-    st->graph_exec = nullptr;
-    st->graph = nullptr;
-    st->graph_key = -1;
+void drop_graph(NbState::EvalGraph& G) {
+    if (G.exec) cudaGraphExecDestroy(G.exec);
+    if (G.graph) cudaGraphDestroy(G.graph);
+    G.exec = nullptr;
+    G.graph = nullptr;
+    G.key = -1;
+}
+
+void drop_graphs(NbState* st) {
+    for (NbState::EvalGraph& G : st->eval_graph) drop_graph(G);
 }
 
 // Everything the captured launches depend on besides the device buffers' contents.
@@ -1000,17 +1007,17 @@ long long launch_key(const NbState* st) {
 int launch_kernels(NbState* st) {
     if (!st->use_graph) return issue_kernels(st);
     const long long key = launch_key(st);
-    if (st->graph_exec != nullptr && st->graph_key == key) {
-        CU(cudaGraphLaunch(st->graph_exec, st->stream));
+    NbState::EvalGraph& G = st->eval_graph[use_cells(st, st->stepping, host_slots(st)) ? 1 : 0];
+    if (G.exec != nullptr && G.key == key) {
+        CU(cudaGraphLaunch(G.exec, st->stream));
         note_evaluation(st, false, st->stepping, true);
         return 0;
     }
-    if (st->prepared_key != key) {
-        drop_graph(st);
-        st->prepared_key = key;
+    drop_graph(G);
+    if (G.prepared != key) {
+        G.prepared = key;
         return issue_kernels(st);
     }
-    drop_graph(st);
     CU(cudaStreamBeginCapture(st->stream, cudaStreamCaptureModeThreadLocal));
     st->capturing = true;
     int rc = issue_kernels(st);
@@ -1022,10 +1029,10 @@ int launch_kernels(NbState* st) {
         return rc;
     }
     CU(end);
-    st->graph = g;
-    CU(cudaGraphInstantiate(&st->graph_exec, g, 0));
-    st->graph_key = key;
-    CU(cudaGraphLaunch(st->graph_exec, st->stream));
+    G.graph = g;
+    CU(cudaGraphInstantiate(&G.exec, g, 0));
+    G.key = key;
+    CU(cudaGraphLaunch(G.exec, st->stream));
     note_evaluation(st, false, st->stepping, true);
     return 0;
 }
@@ -1120,7 +1127,7 @@ void state_free(NbState* st) {
     for (NbState* g : st->groups) state_free(g);
     st->groups.clear();
     cudaSetDevice(st->device);
-    drop_graph(st);
+    drop_graphs(st);
     res_free(st);
     void* dev[] = {st->d_xq, st->d_pid, st->d_keys, st->d_force, st->d_cstart, st->d_ccount, st->d_cmask,
                    st->d_cscale, st->d_acc, st->d_cell_epot, st->d_tasks, st->d_tshift, st->d_coef, st->d_potinfo,
@@ -1593,7 +1600,7 @@ int st_setstream(NbState* st, void* stream) {
     CU(cudaSetDevice(st->device));
     CU(cudaStreamSynchronize(st->stream));
     cudaStream_t s = stream ? static_cast<cudaStream_t>(stream) : st->own_stream;
-    if (s != st->stream) drop_graph(st);
+    if (s != st->stream) drop_graphs(st);
     st->stream = s;
     return 0;
 }
@@ -2973,8 +2980,8 @@ extern "C" int engine_cuda_graph(struct engine* e, int enable) {
     if (e == nullptr || e->cuda == nullptr) return engine_err_null;
     NbState* st = state(e);
     st->use_graph = enable != 0;
-    if (!st->use_graph) drop_graph(st);
-    st->prepared_key = -1;
+    if (!st->use_graph) drop_graphs(st);
+    for (NbState::EvalGraph& G : st->eval_graph) G.prepared = -1;
     return 0;
 }
 
@@ -3504,8 +3511,8 @@ extern "C" int engine_batch_graph(struct engine_batch* b, int enable) {
     if (b == nullptr) return engine_err_null;
     NbState* st = bstate(b);
     st->use_graph = enable != 0;
-    if (!st->use_graph) drop_graph(st);
-    st->prepared_key = -1;
+    if (!st->use_graph) drop_graphs(st);
+    for (NbState::EvalGraph& G : st->eval_graph) G.prepared = -1;
     return 0;
 }
 

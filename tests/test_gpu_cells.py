@@ -447,3 +447,23 @@ def test_the_autotuners_time_is_an_evaluations():
         t.append(b.kernel_times()[0])
     assert 0.9 * np.median(t) < ms < 1.1 * np.median(t), (ms, t)
     b.close()
+
+
+def test_alternating_forms_replay_a_graph_each():
+    """Force evaluations (cell form) and host-threaded steps (queue form) of one engine in turn: each
+    is captured at its second launch and replayed from then on (the steps are too short for a
+    particle to change cells)."""
+    sysm = chain_mix()
+    sysm.dt = 1e-9
+    out = []
+    for graph in (True, False):
+        e = M.Engine.from_system(sysm)
+        e.graph(graph)
+        for k in range(4):
+            e.nonbond()
+            assert e.form() == ("cells", 24, graph and k > 0)
+            e.step_host()
+            assert e.form() == ("queue", 0, graph and k > 0)
+        out.append(e.parts())
+        e.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
