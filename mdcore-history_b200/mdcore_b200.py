@@ -219,6 +219,9 @@ def _check(rc: int, what: str):
     if rc is not None and rc < 0:
         import io, tempfile
         libc = C.CDLL(None)
+        # a FILE* is a pointer: the default int would cut it to 32 bits
+        libc.fdopen.restype, libc.fdopen.argtypes = C.c_void_p, [C.c_int, C.c_char_p]
+        libc.fflush.argtypes = libc.fclose.argtypes = [C.c_void_p]
         msg = ""
         with tempfile.TemporaryFile(mode="w+") as tf:
             fp = libc.fdopen(os.dup(tf.fileno()), b"w")

@@ -3,6 +3,8 @@ every function its header declares, builds bit-identical potential tables, bins 
 like the reference and refuses what it does not implement."""
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -150,3 +152,26 @@ def test_headers_compile_cleanly(std, tmp_path):
                         "-I" + os.path.join(ROOT, "include"), str(src), "-o", str(tmp_path / "inc.o")],
                        capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stderr
+
+
+def test_errors_are_reported_from_any_thread():
+    """The error text is written through a C stream, whose address has 64 bits (on a thread's own
+    heap it lies above 4 GB; cut to 32 it crashed the process)."""
+    code = """
+import threading
+import numpy as np
+import mdcore_b200 as M
+out = []
+def fail():
+    try:
+        M.Engine(np.zeros(3), np.full(3, 0.1), np.ones(3), 1.0)
+    except M.MdcoreError as x:
+        out.append(str(x))
+t = threading.Thread(target=fail)
+t.start()
+t.join()
+assert len(out) == 1 and "space_init" in out[0] and "engine_init" in out[0], out
+"""
+    env = dict(os.environ, PYTHONPATH=os.path.dirname(M.__file__))
+    r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, (r.returncode, r.stderr)
