@@ -742,11 +742,15 @@ __global__ void __launch_bounds__(kCellWarps * 32 + 32, 1) sweep_cells(CellParam
 }
 
 namespace {
+// Shared memory of a block at most (the attribute of all launches, as kSweepSmem).
+constexpr size_t kCellSmem = 227 * 1024;
+
 template <bool EX, int TAB, int ROWS>
 cudaError_t launch_k(const CellParams& C, int nw, size_t smem, int grid, bool capturing, cudaStream_t s) {
     auto kern = sweep_cells<EX, TAB, ROWS>;
     if (!capturing) {
-        const cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t err =
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCellSmem);
         if (err != cudaSuccess) return err;
     }
     kern<<<grid, nw * 32, smem, s>>>(C);
@@ -776,7 +780,7 @@ size_t cell_units_bound(size_t nslots, int ncells, int cap, int maxtasks) {
 // 8 copies (no bank conflicts) up to 32 KB of tables, fewer for larger ones; as many warps, up
 // to kCellWarps, as the rest of an SM's 227 KB holds.
 bool cell_sweep_shape(int rows, int ncoef, int npots, int mt, int* nw, int* copies, size_t* smem) {
-    const size_t room = 227 * 1024, slice = rows == 24 ? sizeof(CellWarp<24>) : sizeof(CellWarp<32>);
+    const size_t room = kCellSmem, slice = rows == 24 ? sizeof(CellWarp<24>) : sizeof(CellWarp<32>);
     auto tables = [&](int n) { return (size_t)ncoef * 4 * n + (size_t)npots * 16 + (size_t)((mt * mt + 3) & ~3) * 4; };
     *copies = 8;
     while (*copies > 1 && tables(*copies) > 32 * 1024) *copies /= 2;

@@ -567,10 +567,15 @@ int chunk_events(NbState* st, size_t n) {
     return 0;
 }
 
+// Shared memory of a queue or plain sweep's block at most.  The kernels' attribute is set to this
+// and not to a launch's own size: it is one for all engines of the process, and a smaller one set
+// by another engine (or thread) refused launches that were captured, or issued, after it.
+constexpr size_t kSweepSmem = 220 * 1024;
+
 template <int NW>
 int launch_plain_nw(NbState* st, const Params& P, int cap, size_t smem) {
     if (!st->capturing)
-        CU(cudaFuncSetAttribute(sweep_tasks<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CU(cudaFuncSetAttribute(sweep_tasks<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem));
     sweep_tasks<NW><<<st->ntasks, NW * 32, smem, st->stream>>>(P, cap);
     CU(cudaGetLastError());
     return 0;
@@ -584,7 +589,7 @@ int launch_plain(NbState* st, const Params& P, int cap) {
         nw /= 2;
         smem = sweep_smem_bytes(cap, nw, tc, tp, st->max_type);
     }
-    if (smem > 220 * 1024) {
+    if (smem > kSweepSmem) {
         errs_register(engine_err_maxparts, "Cell too large for the sweep kernel's shared memory.", __LINE__,
                       __func__, __FILE__);
         return engine_err = engine_err_maxparts;
@@ -605,7 +610,7 @@ int launch_tuned_k(NbState* st, const TunedParams& T, int cap, size_t smem) {
     auto kern = LAY ? sweep_tiled<NW, EX, TAB, WIN, STG, TPSM, TINY> : sweep_tuned<NW, EX, TAB, WIN, STG, TPSM, TINY>;
     int grid = st->last_grid;
     if (!st->capturing) {
-        CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem));
         int per_sm = 0;
         CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NW * 32, smem));
         if (per_sm < 1) per_sm = 1;
@@ -689,7 +694,7 @@ int launch_tuned(NbState* st, const Params& P, int cap4) {
         nw /= 2;
         smem = warps_smem_bytes(cap, nw, tc, tp, st->max_type, st->stages);
     }
-    if (smem > 220 * 1024) {
+    if (smem > kSweepSmem) {
         errs_register(engine_err_maxparts, "Cell too large for the sweep kernel's shared memory.", __LINE__,
                       __func__, __FILE__);
         return engine_err = engine_err_maxparts;
@@ -3691,7 +3696,7 @@ int noalloc_sweep_nw(const NbState* st, const TunedParams& T, int cap, size_t sm
     cudaFuncAttributes fa;
     CU(cudaFuncGetAttributes(&fa, kern));
     if (fa.maxDynamicSharedSizeBytes < (int)smem)
-        CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CU(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSweepSmem));
     int per_sm = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NW * 32, smem));
     kern<<<st->sm_count * std::max(1, per_sm), NW * 32, smem, s>>>(T, cap);
@@ -3745,7 +3750,7 @@ int nonbond_noalloc(struct engine* e, const void* xq, const int* pid, const int*
         nw = 2;
         smem = warps_smem_bytes(cap, nw, tc, tp, st->max_type, 1);
     }
-    if (smem > 220 * 1024)
+    if (smem > kSweepSmem)
         return noalloc_fail(engine_err_maxparts, "Cell too large for the sweep kernel's shared memory.", __LINE__);
 
     CU(cudaSetDevice(st->device));

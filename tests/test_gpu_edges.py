@@ -137,3 +137,32 @@ def test_far_exclusions_use_the_list():
     err = force_errors(f, o["f"])
     assert err["global_rel"] <= 2e-6, err
     e.close()
+
+
+@pytest.mark.parametrize("form", ["queue", "tiled", "plain", "cells"])
+def test_engines_of_different_table_sizes_capture_side_by_side(form, monkeypatch):
+    """Two engines run one kernel with different amounts of shared memory (their tables' sizes):
+    the launches of one neither refuse those captured nor those replayed by the other."""
+    monkeypatch.setenv("MDB_SWEEP_FORM", "cells" if form == "cells" else "queue")
+    engines, want = [], []
+    for tol in (1e-5, 1e-3, 1e-4, 1e-5):
+        sysm = W.water_spce(10, seed=1, tol=tol)
+        for graph in (False, True):
+            e = M.Engine.from_system(sysm)
+            e.graph(graph)
+            if form == "tiled":
+                e.set_layout(1)
+            e.tune(0, plain=form == "plain")
+            if graph:
+                engines.append(e)
+            else:
+                e.nonbond()
+                want.append(e.forces())
+                e.close()
+    for k in range(4):
+        for e, f in zip(engines, want):
+            e.nonbond()
+            assert e.form().graph == (k > 0)
+            assert np.array_equal(e.forces(), f)
+    for e in engines:
+        e.close()
