@@ -316,6 +316,14 @@ int dev_alloc(T** p, size_t n) {
     return 0;
 }
 
+// Uploads and clears of set-up run on the legacy stream, for which the engines' streams (and a
+// caller's non-blocking one) do not wait, and a copy from pageable memory may return before it has
+// landed: whoever has issued some waits here before anything is launched on them.
+int settle_uploads() {
+    CU(cudaStreamSynchronize(cudaStreamLegacy));
+    return 0;
+}
+
 // (Re)allocates the per-particle buffers for `ncap` slots.
 int alloc_particles(NbState* st, int ncap) {
     if (ncap <= st->ncap) return 0;
@@ -336,8 +344,8 @@ int alloc_particles(NbState* st, int ncap) {
     CU(cudaMallocHost(&st->h_force, sizeof(unsigned long long) * 3 * ncap));
     cudaFree(st->d_forcef);
     if (dev_alloc(&st->d_forcef, 3 * (size_t)ncap)) return engine_err_cuda;
-    CU(cudaMemset(st->d_xq, 0, sizeof(float4) * ncap));
-    CU(cudaMemset(st->d_pid, 0, sizeof(int) * ncap));
+    CU(cudaMemsetAsync(st->d_xq, 0, sizeof(float4) * ncap, st->stream));     // before the uploads
+    CU(cudaMemsetAsync(st->d_pid, 0, sizeof(int) * ncap, st->stream));
     st->ncap = ncap;
     return 0;
 }
@@ -789,7 +797,7 @@ int build_cell_tasks(NbState* st) {
     CU(cudaMemcpy(st->d_ctasks, ct.data(), sizeof(TaskRec) * nt, cudaMemcpyHostToDevice));
     CU(cudaMemcpy(st->d_cshift, cs.data(), sizeof(float4) * nt, cudaMemcpyHostToDevice));
     CU(cudaMemcpy(st->d_toff, toff.data(), sizeof(int) * toff.size(), cudaMemcpyHostToDevice));
-    return 0;
+    return settle_uploads();
 }
 
 // Room for the units of `slots` particle slots in cells of at most cap4, grown on a direct
@@ -1428,7 +1436,7 @@ int load_state(NbState* st) {
         if (rc == 0) rc = reserve_units(st, slots, (std::min(most, kMaxPartsPerCell) + 3) & ~3);
         if (rc < 0) return rc;
     }
-    return 0;
+    return settle_uploads();
 }
 
 // Charges by global particle id from the engines' host cells, to the device (explicit
@@ -2125,7 +2133,8 @@ int res_alloc(NbState* st, int capc, int mcap, long long n) {
     CU(cudaMemcpy(st->r_engine_imass, imass.data(), sizeof(double) * imass.size(), cudaMemcpyHostToDevice));
     st->up_aux.assign((size_t)n + 1, NbState::UpAux{0, 0.f, 0, 0, 0});
     st->res_active = true;
-    return res_build_bonds(st);
+    const int rc = res_build_bonds(st);
+    return rc < 0 ? rc : settle_uploads();
 }
 
 // Pipeline chunks of an engine_step transfer of np particles, 1 to st->max_chunks (8; fewer
@@ -2253,7 +2262,7 @@ int elog_restart(NbState* st) {
     const unsigned long long zero = 0ull;
     CU(cudaMemset(st->r_elog, 0, sizeof(unsigned long long) * 4 * (size_t)st->elog_cap));
     CU(cudaMemcpy(st->r_eacc + 1, &zero, sizeof(zero), cudaMemcpyHostToDevice));
-    return 0;
+    return settle_uploads();
 }
 
 // The launches of one resident step: re-binning into the other side, the force evaluation,
@@ -2527,6 +2536,8 @@ int st_resident_steps(NbState* st, int nsteps) {
         if (st->elog_cap > 0) {       // the log keeps counting from the steps already done
             const unsigned long long base = (unsigned long long)done;
             CU(cudaMemcpy(st->r_eacc + 1, &base, sizeof(base), cudaMemcpyHostToDevice));
+            rc = settle_uploads();
+            if (rc < 0) return rc;
         }
     }
     return 0;
@@ -2875,13 +2886,9 @@ extern "C" int engine_cuda_setspin(struct engine* e, int polls) {
     CU(cudaSetDevice(st->device));
     CU(cudaStreamSynchronize(st->stream));
     CU(cudaMemcpyToSymbol(c_spin_limit, &v, sizeof(v)));
-    return 0;
+    return settle_uploads();
 }
 
-// Test hook of the failure path: with enable = 1 the sweeps on the engine's device neither
-// arrive on their staging mbarriers nor issue a copy, so every wait runs out after the spin
-// limit, the evaluation fails with engine_err_cuda ("Bulk copy into shared memory timed
-// out.") and nothing is in flight; 0 restores normal copies.
 // Test hook: lower limits of the cell form (0: its own), units of an evaluation and particle
 // slots of one that runs in it.
 extern "C" int engine_cuda_celllimits_test(struct engine* e, int units, int slots) {
@@ -2895,6 +2902,10 @@ extern "C" int engine_cuda_celllimits_test(struct engine* e, int units, int slot
     return 0;
 }
 
+// Test hook of the failure path: with enable = 1 the sweeps on the engine's device neither
+// arrive on their staging mbarriers nor issue a copy, so every wait runs out after the spin
+// limit, the evaluation fails with engine_err_cuda ("Bulk copy into shared memory timed
+// out.") and nothing is in flight; 0 restores normal copies.
 extern "C" int engine_cuda_copytimeout_test(struct engine* e, int enable) {
     if (e == nullptr || e->cuda == nullptr) return engine_err_null;
     if (enable != 0 && enable != 1) return engine_err_range;
@@ -2903,7 +2914,7 @@ extern "C" int engine_cuda_copytimeout_test(struct engine* e, int enable) {
     CU(cudaStreamSynchronize(st->stream));
     CU(cudaMemcpyToSymbol(c_skip_copies, &enable, sizeof(enable)));
     if (st->device >= 0 && st->device < kHookDevices) copy_hook[st->device].store(enable);
-    return 0;
+    return settle_uploads();
 }
 
 extern "C" int engine_cuda_setaccum(struct engine* e, int fp32) {
@@ -2950,7 +2961,7 @@ extern "C" int engine_cuda_energylog(struct engine* e, int cap) {
             st->res_active ? (unsigned long long)(st->res_done_total + st->res_done) : 0ull;
         CU(cudaMemcpy(st->r_eacc + 1, &base, sizeof(base), cudaMemcpyHostToDevice));
     }
-    return 0;
+    return settle_uploads();
 }
 
 // The records of the log in step order: out[4 k + 0..3] = resident step number (1 = the
@@ -3600,7 +3611,7 @@ int st_setorder(NbState* st, const int* order, int n) {
     // An order is about the task queue.  Given after the autotuner it selects the queue form
     // (in its best shape); before it, the form (and so the rounding of the forces) stays.
     if (st->tuned) st->queue_form = true;
-    return 0;
+    return settle_uploads();
 }
 }  // namespace
 
@@ -3952,7 +3963,7 @@ SchedState* sched(struct engine* e, NbState* st) {
     if (bad) return nullptr;
     cudaMemset(ss->d_dur, 0, sizeof(double) * n);
     cudaMemset(ss->d_nrec, 0, sizeof(int) * n);
-    return ss;
+    return settle_uploads() < 0 ? nullptr : ss;
 }
 
 }  // namespace
@@ -4052,6 +4063,7 @@ extern "C" int engine_sched_targets(struct engine* e, float* targets_out, int n)
     std::vector<float> tg(st->ntasks);
     for (int t = 0; t < st->ntasks; t++) tg[t] = nrec[t] > 0 ? (float)(dur[t] / nrec[t] / mean) : 0.f;
     CU(cudaMemcpy(ss->d_target, tg.data(), sizeof(float) * st->ntasks, cudaMemcpyHostToDevice));
+    if (settle_uploads() < 0) return engine_err_cuda;
     if (targets_out != nullptr) {
         if (n != st->ntasks) return engine_err_range;
         std::copy(tg.begin(), tg.end(), targets_out);
@@ -4082,6 +4094,7 @@ extern "C" int engine_sched_train(struct engine* e, int epochs, int batch, float
         CU(cudaMemcpy(ss->d_wm, w.data(), sizeof(float) * NB_MLP_NPARAM, cudaMemcpyHostToDevice));
         CU(cudaMemset(ss->d_m, 0, sizeof(float) * NB_MLP_NPARAM));
         CU(cudaMemset(ss->d_v, 0, sizeof(float) * NB_MLP_NPARAM));
+        if (settle_uploads() < 0) return engine_err_cuda;
         if (nb_mlp_round(ss->d_wm, ss->d_wb, st->stream) < 0) return engine_err_cuda;
     }
     const int n = st->ntasks;

@@ -727,6 +727,9 @@ int build(struct engine* e, RigidDev* rd) {
     CU(cudaMallocHost(&rd->h_xp, sizeof(double) * 3 * ns));
     CU(cudaMallocHost(&rd->h_stat, sizeof(int) * 2));
     rd->h_stat[0] = rd->h_stat[1] = 0;
+    // a copy from pageable memory may return before it has landed, and the engines' streams do not
+    // wait for the legacy stream
+    CU(cudaStreamSynchronize(cudaStreamLegacy));
     rd->gen = e->rigids_gen;
     return 0;
 }
