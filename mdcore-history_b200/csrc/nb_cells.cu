@@ -680,10 +680,11 @@ __global__ void __launch_bounds__(kCellWarps * 32 + 32, 1) sweep_cells(CellParam
                 const float gx = fmaxf(fmaxf(lox - x, x - hix), 0.f), gy = fmaxf(fmaxf(loy - y, y - hiy), 0.f),
                             gz = fmaxf(fmaxf(loz - z, z - hiz), 0.f);
                 const float nj = fmaf(z, z, fmaf(y, y, x * x));
-                const bool far = !(nj < INFINITY) ||
-                                 fmaf(gz, gz, fmaf(gy, gy, gx * gx)) > fmaf(kSlack, nj + nimax, sh.w);
-                const unsigned ball = __ballot_sync(FULL, on && !far);
-                if (on && !far) {
+                // no less than: the slack covers equality, and neither side of a non-finite position
+                // (both infinite, or the right one NaN) is less than the other
+                const bool close = on && fmaf(gz, gz, fmaf(gy, gy, gx * gx)) < fmaf(kSlack, nj + nimax, sh.w);
+                const unsigned ball = __ballot_sync(FULL, close);
+                if (close) {
                     const int o = (b0 + nb + __popc(ball & ((1u << lane) - 1u))) & (kCellRing - 1);
                     W.bx[o] = xj;
                     W.bm[o] = meta;
