@@ -410,9 +410,13 @@ def timed_resident_steps(tgt, stream, flush, steps, torch):
     return tot / steps, sweep / steps, info.pairs - p0
 
 
-def read_traffic(workload):
-    """dram read + write bytes of one sweep launch, from the committed ncu summary."""
-    prof = os.path.join(ROOT, "profiles", WORKLOADS[workload][2])
+def read_traffic(workload, form):
+    """dram read + write bytes of one sweep launch in that form, from the committed ncu summary
+    (None where there is none)."""
+    name = WORKLOADS[workload][2]
+    if form == "cells":
+        name = name.replace("sweep_", "sweep_cells_", 1)
+    prof = os.path.join(ROOT, "profiles", name)
     if os.path.exists(prof):
         for ln in open(prof):
             if ln.startswith("dram_bytes_per_launch"):
@@ -420,20 +424,22 @@ def read_traffic(workload):
     return None
 
 
-def launch_obj(warps, layout, stages, occupancy, tune_ms):
-    return {"warps_per_block": warps, "lanes": "8i x 4j" if layout else "32i", "staging_buffers": stages,
+def launch_obj(warps, layout, stages, occupancy, tune_ms, form):
+    if form.name == "cells":             # the shape returned is the queue form's best
+        return {"form": "cells", "rows_per_unit": form.rows, "autotune_ms": tune_ms, "cuda_graph": True}
+    return {"form": form.name, "warps_per_block": warps, "lanes": "8i x 4j" if layout else "32i", "staging_buffers": stages,
             "threads_per_sm": occupancy, "autotune_ms": tune_ms, "cuda_graph": True}
 
 
-def roofline_obj(M, local_rank, pairs, sweep_ms, layout, workload):
+def roofline_obj(M, local_rank, pairs, sweep_ms, layout, workload, form):
     peak = M.fp32_peak_tflops(local_rank)
     achieved = FLOPS_PER_PAIR * pairs / (sweep_ms * 1e-3) / 1e12
     return {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-            "traffic": read_traffic(workload),      # of the queue form's sweep
-            # one table: the autotuner may keep the cell form (sweep_cells) instead
-            "kernel": ("sweep_tiled" if layout else "sweep_tuned")
-                      + (" or sweep_cells, the faster" if workload in ("replicas", "argon") else ""),
-            "kernel_ms": sweep_ms, "flops_per_pair": FLOPS_PER_PAIR,
+            "traffic": read_traffic(workload, form.name),
+            "kernel": "sweep_cells" if form.name == "cells" else "sweep_tiled" if layout else "sweep_tuned",
+            "kernel_ms": sweep_ms,
+            # the cell form's candidate count (every step here: one per call) shares the SMs meanwhile
+            "beside": "count_candidates" if form.name == "cells" else None, "flops_per_pair": FLOPS_PER_PAIR,
             "peak_source": "measured FP32 FMA loop on this GPU (engine_cuda_fp32_peak); "
                            "MEASURED_PEAKS.json has no FP32 figure"}
 
@@ -495,6 +501,7 @@ def measure(workload, args, rank, world, local_rank, dist, with_cpu):
     # ---- force evaluation alone (sort + sweep), resident and with host buffers
     barrier()
     fe_ms, fe_sweep = timed_force_evals(tgt, stream, flush, args.steps, torch)
+    fe_form = tgt.form()
     barrier()
     tgt.unload_parts()
     fe_e2e = 0.0
@@ -538,6 +545,7 @@ def measure(workload, args, rank, world, local_rank, dist, with_cpu):
         tgt.resident_steps(max(args.warmup, 25 if rigid else 3))     # past the P-SHAKE refinement steps
         barrier()
         ms, ms_sweep, pairs_timed = timed_resident_steps(tgt, stream, flush, args.steps, torch)
+        step_form = tgt.form()
         barrier()
         pairs = pairs_timed / args.steps
         tgt.resident_sync()
@@ -611,7 +619,12 @@ def measure(workload, args, rank, world, local_rank, dist, with_cpu):
         parallelism = (f"replicas round-robin over {world} GPUs ({len(systems)} on rank 0)" if share
                        else f"replicas x{world}")
         setup = {"tasks": tgt.ntasks(), "cells": ncells, "candidates_per_step": int(st.candidates),
-                 "launch": launch_obj(warps, layout, stages, occupancy, tune_ms)}
+                 "launch": launch_obj(warps, layout, stages, occupancy, tune_ms, fe_form if force_only else step_form)}
+        # device kernels of one evaluation: the cell form's unit list, sweep and candidate count, or
+        # the sort, the queue compaction (3, systems with empty cells) and the sweep
+        sort_sweep = {form: ("unit list, sweep_cells, candidate count" if form.name == "cells" else "sort, sweep")
+                      for form in (fe_form, fe_form if force_only else step_form)}
+        launches = {form: 3 if form.name == "cells" else 2 + 3 * int(compact) for form in sort_sweep}
         if force_only:
             slots = sum(int((((cell_counts(s, e) + 3) // 4) * 4).sum()) for s, e in zip(systems, engines))
             fe_h2d, fe_d2h = 20 * slots + 4 * (2 * ncells + 1), 12 * slots + 16 * ncells + 64
@@ -620,27 +633,25 @@ def measure(workload, args, rank, world, local_rank, dist, with_cpu):
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": fe_ms, "higher_is_better": True,
                 "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic", "ns_per_day": None,
                 "config": config, "parallelism": parallelism,
-                "step": "one force evaluation: sort + sweep (engine_nonbond_cuda_resident)", "setup": setup,
+                "step": f"one force evaluation: {sort_sweep[fe_form]} (engine_nonbond_cuda_resident)", "setup": setup,
                 "e2e": {"value": world * pairs / (fe_e2e * 1e-3), "unit": UNIT, "ms_per_step": fe_e2e,
                         "h2d_bytes_per_step": fe_h2d, "d2h_bytes_per_step": fe_d2h,
                         "what": "engine_nonbond_cuda with host buffers: positions and ids up, forces and "
                                 "energies down"},
-                "roofline": roofline_obj(M, local_rank, pairs, fe_sweep, layout, workload),
+                "roofline": roofline_obj(M, local_rank, pairs, fe_sweep, layout, workload, fe_form),
                 "plain": {"value": world * pairs / (plain_ms * 1e-3), "ms_per_step": plain_ms,
                           "sweep_ms": plain_sweep,
                           "what": "plain form: one block per task, IEEE sqrt/div, per-step warp reductions"},
-                "gpu_launches": (2 + 3 * int(compact)) * args.steps,
+                "gpu_launches": launches[fe_form] * args.steps,
                 "clocks": clk,
             }
         else:
-            # kernels of one resident step: re-binning (2), sort, queue compaction (3, systems
-            # with empty cells), sweep, integration, constraints (rigid, one per engine)
-            # (the update runs inside the constraint kernel when every particle of a single
-            # system is in a rigid group); the cell form, when the autotuner keeps it, launches one
-            # more (its unit list, sweep and candidate count for sort and sweep), not counted here
+            # kernels of one resident step: re-binning (2), the evaluation's, integration,
+            # constraints (rigid, one per engine; the update runs inside the constraint kernel when
+            # every particle of a single system is in a rigid group)
             fused = (rigid and len(systems) == 1 and
                      len(set(np.asarray(systems[0].rigid)[:, :2].astype(int).ravel().tolist())) == systems[0].n)
-            per_step = 2 + 1 + 3 * int(compact) + 1 + int(not fused) + int(rigid) * len(engines)
+            per_step = 2 + launches[step_form] + int(not fused) + int(rigid) * len(engines)
             line = {
                 "metric": METRIC, "value": pairs_all / (ms * 1e-3), "unit": UNIT, "n_gpus": world,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
@@ -648,7 +659,7 @@ def measure(workload, args, rank, world, local_rank, dist, with_cpu):
                 "ns_per_day": ns_per_day(ms, dt_fs),
                 "config": config, "parallelism": parallelism,
                 "pairs_per_step_timed": pairs_all,
-                "step": "engine_step on the device: re-binning, sort, sweep, integration"
+                "step": f"engine_step on the device: re-binning, {sort_sweep[step_form]}, integration"
                         + (", P-SHAKE" if rigid else "") + "; one CUDA graph per step"
                         + ("; Verlet skin (re-binning and sort only on rebuild steps)" if args.verlet else ""),
                 "setup": setup,
@@ -657,7 +668,7 @@ def measure(workload, args, rank, world, local_rank, dist, with_cpu):
                         "d2h_bytes_per_step": d2h, "host_ms": {k: round(v, 4) for k, v in host.items()},
                         "what": "engine_step (engine_batch_step for the replicas) with the host cells as input "
                                 "and output every step"},
-                "roofline": roofline_obj(M, local_rank, pairs, ms_sweep, layout, workload),
+                "roofline": roofline_obj(M, local_rank, pairs, ms_sweep, layout, workload, step_form),
                 "plain": {"value": plain_all / (plain_ms * 1e-3), "ms_per_step": plain_ms,
                           "sweep_ms": plain_sweep,
                           "what": "the same resident steps with the plain sweep: one block per task, IEEE "
@@ -667,7 +678,7 @@ def measure(workload, args, rank, world, local_rank, dist, with_cpu):
                                       "and constraints through host buffers"},
                 "force_eval": {"value": fe_all / (fe_ms * 1e-3), "ms_per_step": fe_ms, "sweep_ms": fe_sweep,
                                "e2e": {"value": fe_all / (fe_e2e * 1e-3), "ms_per_step": fe_e2e},
-                               "what": "sort + sweep alone at the initial positions (engine_nonbond_cuda_resident; "
+                               "what": f"{sort_sweep[fe_form]} alone at the initial positions (engine_nonbond_cuda_resident; "
                                        "e2e: engine_nonbond_cuda with host buffers)"},
                 "gpu_launches": per_step * args.steps,
                 "clocks": clk,
@@ -997,19 +1008,20 @@ def profile_steps(args):
     else:
         engines = [M.Engine.from_system(built, flags=args.engine_flags, device=0)]
         tgt = engines[0]
-    warps, layout, stages, occupancy = (int(v) for v in ((args.launch or "8,1,1") + ",1024").split(",")[:4])
-    tgt.tune(warps)
-    tgt.set_layout(layout, stages, occupancy)
+    if args.launch or "cells" not in os.environ.get("MDB_SWEEP_FORM", ""):      # a shape: the queue form
+        warps, layout, stages, occupancy = (int(v) for v in ((args.launch or "8,1,1") + ",1024").split(",")[:4])
+        tgt.tune(warps)
+        tgt.set_layout(layout, stages, occupancy)
     tgt.graph(True)
     tgt.resident_begin()
     tgt.resident_steps(args.profile_steps)
     tgt.resident_sync()
-    status = tgt.stats().status
+    status, form = tgt.stats().status, tgt.form()
     tgt.resident_end()
     if status != 0:
         raise SystemExit(f"bench.py: device status {status}")
     print(json.dumps({"profile_steps": args.profile_steps, "workload": args.workload,
-                      "launch": [warps, layout, stages, occupancy], "status": status}))
+                      "form": form.name, "status": status}))
 
 
 def main():

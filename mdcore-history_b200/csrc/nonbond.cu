@@ -744,6 +744,16 @@ bool cell_shape(const NbState* st, int* nw, int* copies, size_t* smem) {
                             smem);
 }
 
+// Records an event; inside a stream capture as an external record node, so that replaying
+// the graph records it again (a plain record would stay internal to the graph).
+int record_event(NbState* st, cudaEvent_t ev) {
+    if (st->capturing)
+        CU(cudaEventRecordWithFlags(ev, st->stream, cudaEventRecordExternal));
+    else
+        CU(cudaEventRecord(ev, st->stream));
+    return 0;
+}
+
 // The cell form's launches on the state's stream: the units of the cells' current counts and
 // their sweep, and beside the sweep, on a stream of its own that forks and joins here, the
 // candidate count (skipped on the device while *count_cand is 0).
@@ -768,6 +778,8 @@ int launch_cells(NbState* st, const Params& P, const int* count_cand) {
     CU(launch_cell_sweep(C, st->ncells, st->cell_rows, st->d_units, st->has_excl,
                          st->tab_global ? kTabGlobal : st->one_pot ? kTabOne : kTabShared, nw, smem, st->sm_count,
                          st->capturing, st->stream));
+    const int rc = record_event(st, st->evs1);     // the sweep's end; the count's does not matter
+    if (rc < 0) return rc;
     CU(launch_cell_count(C, st->sm_count, st->side_stream));
     CU(cudaEventRecord(st->ev_join, st->side_stream));
     CU(cudaStreamWaitEvent(st->stream, st->ev_join, 0));
@@ -815,16 +827,6 @@ int reserve_units(NbState* st, size_t slots, int cap4) {
     if (dev_alloc(&st->d_units, need)) return engine_err_cuda;
     st->units_cap = need;
     ++st->buf_gen;
-    return 0;
-}
-
-// Records an event; inside a stream capture as an external record node, so that replaying
-// the graph records it again (a plain record would stay internal to the graph).
-int record_event(NbState* st, cudaEvent_t ev) {
-    if (st->capturing)
-        CU(cudaEventRecordWithFlags(ev, st->stream, cudaEventRecordExternal));
-    else
-        CU(cudaEventRecord(ev, st->stream));
     return 0;
 }
 
@@ -960,7 +962,7 @@ int issue_kernels(NbState* st, const DevView& V, bool span = true) {
     else
         rc = st->plain ? launch_plain(st, P, cap) : launch_tuned(st, P, cap);
     if (rc < 0) return rc;
-    rc = record_event(st, st->evs1);
+    if (!cells) rc = record_event(st, st->evs1);
     if (rc < 0) return rc;
     if (f32) {
         const size_t n = 3 * V.slots;
