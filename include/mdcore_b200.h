@@ -652,7 +652,9 @@ int engine_cuda_setlayout(struct engine *e, int layout, int stages, int occupanc
  * engine_sched_order, engine_sched_apply) selects it.  A shape that is the one returned here
  * (window 4) stands for the autotuner's choice, and giving it brings that choice back.
  * Without the autotuner: the queue form, and for force evaluations of systems whose tables do
- * not fit in shared memory the cell form.  The environment variable MDB_SWEEP_FORM (queue,
+ * not fit in shared memory, of few large cells (80 particles or more on average, up to some 250
+ * cells in all the state's engines), the cell form.  An engine of that kind and a batch of it
+ * can so differ in form, and in the rounding of the forces' sums.  The environment variable MDB_SWEEP_FORM (queue,
  * cells, cells24), read when the device state is built, overrides both, for time steps too. */
 int engine_cuda_autotune(struct engine *e, int reps, int *warps, int *layout, int *stages, int *occupancy,
                          float *ms);

@@ -1333,14 +1333,23 @@ int load_state(NbState* st) {
         size_t smem = 0;
         st->cells_ok = st->max_cell_tasks <= kCellTasks && cell_shape(st, &nw, &copies, &smem) && nw >= 4;
         // Without the autotuner: the cell form (24 rows) where the tables are read from global
-        // memory (many type pairs, explicit charges; force evaluation of solvated chains, 12,400
-        // atoms: sweep 0.55 -> 0.27 ms), else the task queue, which small systems finish sooner (argon, 8,788 atoms:
-        // 0.058 against 0.066 ms).  Properties of the engines' tables, so an engine runs the same
-        // form alone and in a batch.  MDB_SWEEP_FORM=queue, cells or cells24 overrides.
+        // memory (many type pairs, explicit charges) and the queue form's tasks are few and large:
+        // at most 1.25 per worker warp, 80 particles or more per cell on average.  There a task is
+        // one warp's for hundreds of microseconds, while the cell form splits every cell's work.
+        // Force evaluation of solvated chains, device us, queue / cells24, by cells x particles per
+        // cell: 27 x 92 240 / 227, 27 x 138 396 / 279, 64 x 194 709 / 415, 125 x 99 394 / 249,
+        // 125 x 149 519 / 486, 216 x 86 364 / 289, 216 x 158 754 / 588; outside: 27 x 69 166 / 245,
+        // 216 x 36 158 / 186, 343 x 99 368 / 427, 343 x 163 803 / 783, 512 x 133 512 / 840,
+        // 1000 x 34 181 / 296.  With tables in shared memory the queue form: small systems finish
+        // sooner there (argon, 8,788 atoms: 0.058 against 0.066 ms per step).
+        // MDB_SWEEP_FORM=queue, cells or cells24 overrides.
+        long long parts = 0;
+        for (const struct engine* e : st->engines) parts += e->s.nr_parts;
+        const bool few_large = parts >= 80LL * st->ncells && 4LL * ntasks <= 5LL * st->sm_count * (640 / 32);
         const char* form = std::getenv("MDB_SWEEP_FORM");
         st->cells_forced = form && std::strncmp(form, "cells", 5) == 0;
         st->queue_forced = form && !st->cells_forced;
-        st->queue_form = form ? st->queue_forced : !st->tab_global;
+        st->queue_form = form ? st->queue_forced : !(st->tab_global && few_large);
         st->cell_rows = form ? (std::strcmp(form, "cells24") == 0 ? 24 : 32) : st->tab_global ? 24 : 32;
     }
     if (dev_alloc(&st->d_tasks, tasks.size()) || dev_alloc(&st->d_tshift, tshift.size())) return engine_err_cuda;

@@ -142,8 +142,7 @@ def test_candidates_of_the_last_step_of_every_call(monkeypatch):
 def test_steps_of_several_tables_keep_the_queue_form(monkeypatch):
     """Default engines of many tables: force evaluations run the cell form, time steps (device
     and host-threaded) give the queue form's trajectory bit for bit."""
-    sysm = W.chains_water(nchains=6, length=20, nwater=200, box=(4.0, 4.0, 4.0), seed=2, angles_dihedrals=False)
-    sysm.bonds = None
+    sysm = chain_mix()
     out = []
     for form, host in ((None, False), (None, True), ("queue", False)):
         if form:
@@ -161,8 +160,10 @@ def test_steps_of_several_tables_keep_the_queue_form(monkeypatch):
 
 
 def chain_mix():
-    """Many tables, no bonds: force evaluations run the cell form by default, steps the queue form."""
-    s = W.chains_water(nchains=6, length=20, nwater=200, box=(4.0, 4.0, 4.0), seed=2, angles_dihedrals=False)
+    """Many tables, few large cells, no bonds: force evaluations run the cell form by default, steps
+    the queue form."""
+    s = W.chains_water(nchains=6, length=20, nwater=900, box=(4.0, 4.0, 4.0), seed=2, gap=0.3,
+                       angles_dihedrals=False)
     s.bonds = None
     return s
 
@@ -467,3 +468,21 @@ def test_alternating_forms_replay_a_graph_each():
         out.append(e.parts())
         e.close()
     assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("cells, per_cell, form", [(3, 60, "queue"), (3, 100, "cells"), (6, 100, "cells"),
+                                                   (7, 100, "queue")])
+def test_default_form_by_number_and_size_of_cells(cells, per_cell, form):
+    """Tables in global memory: the cell form where the queue form's tasks are few and large."""
+    n = 22 * (cells ** 3 * per_cell // 22)
+    s = W.chains_water(nchains=1, length=22, nwater=0, box=(1.2 * cells + 0.01,) * 3, seed=2, angles_dihedrals=False)
+    rng = np.random.default_rng(1)
+    s.x = rng.uniform(0.0, 1.2 * cells, size=(n, 3))
+    s.type = np.tile(np.arange(22, dtype=np.int32), n // 22)
+    s.q = np.zeros(n)
+    s.excl, s.bonds, s.rigid = np.zeros((0, 2), np.int32), None, None
+    e = M.Engine.from_system(s)
+    e.load_parts()
+    e.resident()
+    assert e.form().name == form
+    e.close()
