@@ -812,8 +812,9 @@ int build_cell_tasks(NbState* st) {
     return settle_uploads();
 }
 
-// Room for the units of `slots` particle slots in cells of at most cap4, grown on a direct
-// launch (a captured one has been preceded by a direct one of the same sizes).
+// Room for the units of `slots` particle slots in cells of at most cap4, grown at the upload or
+// on a direct launch (a captured resident step has been preceded by a direct one of the same
+// sizes), with some to spare.
 int reserve_units(NbState* st, size_t slots, int cap4) {
     const size_t need = cell_units_bound(slots, st->ncells, cap4, st->max_cell_tasks);
     if (need <= st->units_cap) return 0;
@@ -824,8 +825,9 @@ int reserve_units(NbState* st, size_t slots, int cap4) {
     if (st->d_units) CU(cudaFree(st->d_units));
     st->d_units = nullptr;
     st->units_cap = 0;
-    if (dev_alloc(&st->d_units, need)) return engine_err_cuda;
-    st->units_cap = need;
+    const size_t room = need + need / 8;
+    if (dev_alloc(&st->d_units, room)) return engine_err_cuda;
+    st->units_cap = room;
     ++st->buf_gen;
     return 0;
 }
@@ -1491,6 +1493,12 @@ int st_load_parts(NbState* st) {
     }
     const int slots = prepare_slots(st);
     if (slots < 0) return slots;
+    // what the evaluation allocates is allocated here, so that a caller may capture it
+    if (use_cells(st, st->stepping, (size_t)slots)) {
+        int rc = build_cell_tasks(st);
+        if (rc == 0) rc = reserve_units(st, (size_t)slots, (st->maxcount + 3) & ~3);
+        if (rc < 0) return rc;
+    }
     const std::vector<int> bounds = chunk_bounds(st, slots);
     for (size_t q = 0; q + 1 < bounds.size(); q++) {
         const int cb = bounds[q], ce = bounds[q + 1];

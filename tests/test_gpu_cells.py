@@ -486,3 +486,36 @@ def test_default_form_by_number_and_size_of_cells(cells, per_cell, form):
     e.resident()
     assert e.form().name == form
     e.close()
+
+
+@pytest.mark.parametrize("form", ["queue", "cells"])
+def test_evaluation_inside_a_capture_of_the_caller(form, monkeypatch):
+    """Uploaded particles are evaluated without an allocation, whatever has changed since the device
+    state was built, so that a caller can capture the evaluation on its own stream."""
+    torch = pytest.importorskip("torch")
+    if form == "queue":
+        monkeypatch.setenv("MDB_SWEEP_FORM", form)
+    sysm = chain_mix()                                   # steps run the queue form
+    sysm.rigid = None
+    sysm.v = W.maxwell_velocities(sysm, 600.0, seed=3)
+    e = M.Engine.from_system(sysm)
+    most = np.bincount(e.cells()).max()
+    while np.bincount(e.cells()).max() < most + 4:       # larger cells than at first
+        e.resident_begin().resident_steps(5).resident_end()
+    stream = torch.cuda.Stream()
+    e.set_stream(stream.cuda_stream)
+    e.load_parts()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        e.resident()
+    assert e.form() == (form, 24 if form == "cells" else 0, False)
+    g.replay()
+    torch.cuda.synchronize()
+    e.unload_parts()
+    f, pairs = e.forces(), e.stats().pairs
+    e.set_stream(0)
+    e.nonbond()
+    assert np.array_equal(e.forces(), f) and e.stats().pairs == pairs
+    del g
+    e.close()
