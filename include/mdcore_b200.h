@@ -524,8 +524,9 @@ int engine_nonbond_cuda_fresh(struct engine *e);
 int engine_cuda_setstream(struct engine *e, void *stream);
 /* Device time (ms) of the last evaluation: its launches from the first to the last (the
  * zeroing, sort and sweep, in the cell form with the candidate count; after resident steps the
- * whole last step), and the sweep alone (with its queue compaction or unit list).  Events recorded on the launch stream, inside the CUDA graph when one is replayed,
- * so host launch latency is not counted. */
+ * whole last step), and the sweep alone (with its queue compaction or unit list).  Events
+ * recorded on the launch stream, inside the CUDA graph when one is replayed, so host launch
+ * latency is not counted. */
 int engine_cuda_kernel_times(struct engine *e, float *total_ms, float *sweep_ms);
 /* Measured FP32 FMA throughput of a device in TFLOP/s (a register-only FMA loop). */
 int engine_cuda_fp32_peak(int device, float *tflops);

@@ -26,12 +26,21 @@
 // What bounds it: instruction latency and issue.  512 argon replicas (1.45 M atoms, cells of
 // 18-45, 58.8 M pairs): 10.2 warp instructions per pair against the queue form's 19.4, issue
 // slots 60 % busy with 2.75 warps per scheduler (the accumulators limit an SM to 12 or 13
-// warps), shared-memory pipe 50 %, DRAM idle; 0.86 ms per sweep against 1.19 and no sort (0.13);
-// a resident step 1.47 -> 0.94 ms.  About half of the instructions evaluate pairs (two per lane
-// and iteration, 52 % of the lane slots carrying one, counted on the CPU: the two lists by
-// number of rows give that, one list gives 40 %), a quarter tests rows.  Solvated chains, 12,400 atoms, tables in global
-// memory, charges: sweep 0.55 -> 0.27 ms.  On cells of 135 particles (water) it loses, 0.45
-// against 0.28 ms per step: every strip walks the whole neighbourhood again.
+// warps), shared-memory pipe 50 %, DRAM idle (95 MB per launch); 0.86 ms per sweep against 1.19
+// and no sort (0.13); a resident step 1.47 -> 0.95 ms (0.6 % of it for non-finite rows).  About
+// half of the instructions evaluate pairs (two per lane and iteration, 52 % of the lane slots
+// carrying one, counted on the CPU: the two lists by number of rows give that, one list gives
+// 40 %), a quarter tests rows.  Solvated chains, 12,400 atoms, tables in global memory, charges:
+// an evaluation with its candidate count 0.71 -> 0.42 ms.  On cells of 135 particles (water) it
+// loses, 0.45 against 0.28 ms per step: every strip walks the whole neighbourhood again.
+//
+// Precision: a row's force is summed in FP32 over all tasks of its cell, in 32 sums (one per
+// lane) that are added pairwise, and converted to fixed point once per unit; the queue form
+// converts after every cell pair and strip.  Error of the forces against 64 bits, 2-norm, queue
+// (32 i) / queue (8 x 4) / cells / cells24, mean of two seeds in 1e-7: argon 32,000 5.79 / 5.77 /
+// 5.76 / 5.77, water 24,000 6.54 / 6.33 / 6.27 / 6.27, slab 1.25 / 1.25 / 1.23 / 1.23, chains of
+// 12,400 1.52 / 1.58 / 1.38 / 1.44, of 3,720 1.48 / 1.34 / 1.44 / 1.41: never above the larger of
+// the queue form's own two layouts.
 // The tables are held in 8 interleaved copies, one per lane of a quarter warp, so that the
 // 16-byte reads at random intervals meet no bank conflicts.
 #include <algorithm>

@@ -142,7 +142,11 @@ __global__ void __launch_bounds__(256) rebin_split(ResidentCells RC, const float
 // it counts its arrivals, a scan over the group gives their first slot, and it writes them.
 // With slot_of, the slot of every particle id of the cell.  The forces of the occupied slots
 // are zeroed for the step here (nothing reads the others): a memset of the whole blocks wrote
-// every spare slot, nine times the particles' on a slab in its vapour.
+// every spare slot, nine times the particles' on a slab in its vapour.  With a warp per cell a
+// lane reads its direction's leavers one by one where a list of all directions' was read 32 at a
+// time: with many leavers and the zeroing 8.8 -> 10.3 us (rigid water, 98,304 atoms, 3,000 K) and
+// 5.7 -> 6.2 us (argon, 108,000 atoms, 3,000 K), less than the memset's launch took: steps of that
+// water 322.6 -> 320.4 us, with a Verlet skin at 300 K 325.8 -> 324.3.
 template <int G>
 __global__ void __launch_bounds__(256) rebin_gather(ResidentCells RC, const Mover* __restrict__ movers,
                                                     const int* __restrict__ nstay, const int* __restrict__ nmove,

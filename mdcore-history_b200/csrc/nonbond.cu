@@ -716,13 +716,14 @@ constexpr int kHookDevices = 64;
 std::atomic<int> copy_hook[kHookDevices];
 
 // Whether an evaluation runs in the cell form: not when the queue form is asked for (a launch
-// shape, see shape_given, or a queue order given after the autotuner), when per-task clocks are recorded, for
-// the unsorted sweep (its candidates are all pairs) or with a Verlet skin (its keys are kept
-// between steps and bound the sweep).  Time steps (steps) of systems of several tables stay in
-// the queue form: the two forms add a particle's pair forces in another order, and over some
-// hundred steps of such systems (close contacts of a random vapour, truncated charges, the
-// constraint iterations) that last bit grows to per mille of the velocities, as it does
-// between the queue form's own lane layouts; a single table's trajectories keep five digits.
+// shape, see shape_given, or a queue order given after the autotuner), when per-task clocks are
+// recorded, for the unsorted sweep (its candidates are all pairs) or with a Verlet skin (its keys
+// are kept between steps and bound the sweep).  Time steps (steps) of systems of several tables
+// stay in the queue form.  That is a choice: the two forms add a particle's pair forces in another
+// order, and over some hundred steps of such systems (close contacts of a random vapour, truncated
+// charges, the constraint iterations) that last bit grows to per mille of the velocities, no more
+// and no less than between the queue form's own lane layouts, between which the autotuner chooses
+// freely.  A single table's trajectories keep five digits.
 // slots: particle slots of the evaluation (list entries hold kCellSlotBits of a slot's number).
 bool use_cells(const NbState* st, bool steps, size_t slots) {
     if (slots > st->cell_slots) return false;
@@ -740,8 +741,8 @@ size_t res_slots(const NbState* st) { return (size_t)st->ncells * st->capc; }
 
 // Worker warps, table copies and shared memory of the cell form for the state's tables.
 bool cell_shape(const NbState* st, int* nw, int* copies, size_t* smem) {
-    return cell_sweep_shape(st->cell_rows, st->tab_global ? 0 : st->ncoef, st->tab_global ? 0 : st->npots, st->max_type, nw, copies,
-                            smem);
+    return cell_sweep_shape(st->cell_rows, st->tab_global ? 0 : st->ncoef, st->tab_global ? 0 : st->npots,
+                            st->max_type, nw, copies, smem);
 }
 
 // Records an event; inside a stream capture as an external record node, so that replaying
