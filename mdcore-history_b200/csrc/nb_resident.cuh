@@ -52,6 +52,11 @@ template <int G>
 __device__ __forceinline__ int group_cell() {
     return (int)((blockIdx.x * blockDim.x + threadIdx.x) / G);
 }
+// A step already aborted; the whole warp agrees, although other blocks may be setting the word now
+// (lanes that had left would not take part in the others' ballots and shuffles).
+__device__ __forceinline__ bool aborted_warp(const unsigned long long* status) {
+    return __any_sync(0xffffffffu, *(volatile const unsigned long long*)status != 0);
+}
 template <int G>
 __device__ __forceinline__ unsigned group_bits(unsigned ballot) {
     if constexpr (G == 32) return ballot;
@@ -72,7 +77,7 @@ __global__ void __launch_bounds__(256) rebin_split(ResidentCells RC, const float
     constexpr unsigned FULL = 0xffffffffu;
     const int gl = threadIdx.x & (G - 1);
     const int c = group_cell<G>();
-    if (*(volatile unsigned long long*)status != 0) return;
+    if (aborted_warp(status)) return;
     const bool cell = c < RC.ncells;          // the warp's ballots need all its lanes
     const int n = cell ? min(count[c], RC.capc) : 0;
     const size_t base = (size_t)c * RC.capc;
@@ -158,7 +163,7 @@ __global__ void __launch_bounds__(256) rebin_gather(ResidentCells RC, const Move
     constexpr int D = (27 + G - 1) / G;
     const int gl = threadIdx.x & (G - 1);
     const int c = group_cell<G>();
-    if (*(volatile unsigned long long*)status != 0) return;
+    if (aborted_warp(status)) return;
     const bool cell = c < RC.ncells;
     const size_t base = (size_t)c * RC.capc;
     int src[D], nm[D], mine = 0;

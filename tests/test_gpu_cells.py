@@ -4,7 +4,8 @@ as the autotuner otherwise does): pairs, exclusions and the sorted sweep's candi
 exact, energy, virial and forces within the parity bounds of the oracle, at the sizes where
 its strips, lists and masks end (cells of 0 to 90 particles, a cell of 1,000, a vapour, list
 and mask exclusions, many tables), and the same results alone, in a batch,
-resident and through engine_step."""
+resident and through engine_step.  Every test asserts the form that ran; the rules by which it is
+chosen, its limits and its graphs have tests of their own."""
 import ctypes as C
 
 import numpy as np
